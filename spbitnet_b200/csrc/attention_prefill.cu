@@ -1,0 +1,229 @@
+// Causal attention of a prompt chunk: T tokens at positions *d_pos .. *d_pos + T - 1 over the KV cache, as T calls of
+// attention_scores_gpu + softmax_gpu + attention_output_gpu (src/kernels/inference_kernels.cu:241-371) give it.
+//
+// A block takes the G query heads of one KV head and R tiles of 16 tokens, a warp one (head, tile): the 16 tokens are
+// the rows of mma.sync m16n8k16.  K and V go through shared memory in tiles of 64 positions, two in flight, read once
+// for all warps of the block.  Scores, running maximum, sum and output are fp32.  The exponentials enter the second
+// product as the sum of two halves (value and remainder, 22 bits), so nothing is rounded to half that was fp32 before.
+// Tiles of positions start at multiples of 64 whatever the chunk, and a tile past a row's own position leaves the row
+// untouched, so a row's bits do not depend on how a prompt is cut into calls.
+//
+// Bound: the tensor pipe (three products of 16 x 64 x head_dim per warp and tile); a block per (head, token) that walks
+// the positions serially, used before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens
+// at 20 heads of 128, this kernel 73 us.
+#include "fused_ops.cuh"
+
+namespace spb {
+
+namespace {
+
+constexpr int kPaTile = 64;  // positions per K / V tile
+constexpr int kPaRows = 16;  // tokens per warp
+
+__device__ __forceinline__ void pa_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void pa_ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void pa_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pa_pack(__half lo, __half hi) {
+    return static_cast<uint32_t>(__half_as_ushort(lo)) | (static_cast<uint32_t>(__half_as_ushort(hi)) << 16);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(256) prefill_attention_kernel(
+    const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V, __half* __restrict__ out,
+    int T, int num_heads, int G, int R, int max_seq_len, float scale_log2, const int* __restrict__ d_pos) {
+    extern __shared__ __align__(128) uint8_t pa_sm[];  // K tile x 2, V tile x 2
+    constexpr int kRowBytes = HD * 2, kTileBytes = kPaTile * kRowBytes;
+    grid_dep_launch();
+    grid_dep_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nthreads = blockDim.x;
+    const int start = *d_pos;
+    const int kvh = blockIdx.y, head = kvh * G + warp % G;
+    const int btile = (gridDim.x - 1 - blockIdx.x) * R;  // the longest rows first
+    const int tok0 = (btile + warp / G) * kPaRows;       // this warp's tokens
+    const int last = min(T, (btile + R) * kPaRows) - 1;  // the block's last token
+    const int npos = start + last + 1;
+    const int ntiles = (npos + kPaTile - 1) / kPaTile;
+    const uint32_t sm = static_cast<uint32_t>(__cvta_generic_to_shared(pa_sm));
+    const uint8_t* kg = reinterpret_cast<const uint8_t*>(K + static_cast<size_t>(kvh) * max_seq_len * HD);
+    const uint8_t* vg = reinterpret_cast<const uint8_t*>(V + static_cast<size_t>(kvh) * max_seq_len * HD);
+
+    auto load_tile = [&](int j) {  // 16-byte pieces, piece c of row r at c ^ (r & 7); positions past the block's last: zero
+        const uint32_t kb = sm + (j & 1) * kTileBytes, vb = kb + 2 * kTileBytes;
+        for (int i = threadIdx.x; i < kPaTile * (HD / 8); i += nthreads) {
+            const int r = i / (HD / 8), c = i % (HD / 8);
+            const int p = j * kPaTile + r;
+            const uint32_t dst = r * kRowBytes + ((c ^ (r & 7)) << 4);
+            const size_t src = static_cast<size_t>(min(p, npos - 1)) * kRowBytes + c * 16;
+            const int n = p < npos ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kb + dst), "l"(kg + src), "r"(n) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vb + dst), "l"(vg + src), "r"(n) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_tile(0);
+
+    const int g = lane >> 2, t4 = lane & 3;
+    const int ta = min(tok0 + g, T - 1), tb = min(tok0 + g + 8, T - 1);  // rows past the batch repeat its last token
+    const int pa = start + ta, pb = start + tb;
+    uint32_t qf[HD / 16][4];
+    {
+        const uint32_t* qa = reinterpret_cast<const uint32_t*>(Q + (static_cast<size_t>(ta) * num_heads + head) * HD) + t4;
+        const uint32_t* qb = reinterpret_cast<const uint32_t*>(Q + (static_cast<size_t>(tb) * num_heads + head) * HD) + t4;
+#pragma unroll
+        for (int k = 0; k < HD / 16; ++k) {
+            qf[k][0] = qa[k * 8];
+            qf[k][1] = qb[k * 8];
+            qf[k][2] = qa[k * 8 + 4];
+            qf[k][3] = qb[k * 8 + 4];
+        }
+    }
+    float o[HD / 8][4];
+#pragma unroll
+    for (int i = 0; i < HD / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[i][c] = 0.0f;
+    float ma = -INFINITY, mb = -INFINITY, la = 0.0f, lb = 0.0f;
+
+    for (int j = 0; j < ntiles; ++j) {
+        if (j + 1 < ntiles) {
+            load_tile(j + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const uint32_t kb = sm + (j & 1) * kTileBytes, vb = kb + 2 * kTileBytes;
+        if (tok0 < T && j * kPaTile <= start + min(tok0 + kPaRows, T) - 1) {  // else: every position is past the warp's rows
+            float s[kPaTile / 8][4];
+#pragma unroll
+            for (int i = 0; i < kPaTile / 8; ++i)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[i][c] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < HD / 16; ++k)
+#pragma unroll
+                for (int nb = 0; nb < kPaTile / 16; ++nb) {
+                    const int r = nb * 16 + (lane & 7) + ((lane >> 4) << 3), c = 2 * k + ((lane >> 3) & 1);
+                    uint32_t b[4];
+                    pa_ldsm4(b, kb + r * kRowBytes + ((c ^ (r & 7)) << 4));
+                    pa_mma(s[2 * nb], qf[k], b[0], b[1]);
+                    pa_mma(s[2 * nb + 1], qf[k], b[2], b[3]);
+                }
+            float na = ma, nb_ = mb;
+#pragma unroll
+            for (int i = 0; i < kPaTile / 8; ++i) {
+                const int p = j * kPaTile + i * 8 + 2 * t4;
+                s[i][0] = p <= pa ? s[i][0] * scale_log2 : -INFINITY;
+                s[i][1] = p + 1 <= pa ? s[i][1] * scale_log2 : -INFINITY;
+                s[i][2] = p <= pb ? s[i][2] * scale_log2 : -INFINITY;
+                s[i][3] = p + 1 <= pb ? s[i][3] * scale_log2 : -INFINITY;
+                na = fmaxf(na, fmaxf(s[i][0], s[i][1]));
+                nb_ = fmaxf(nb_, fmaxf(s[i][2], s[i][3]));
+            }
+#pragma unroll
+            for (int off = 1; off < 4; off <<= 1) {
+                na = fmaxf(na, __shfl_xor_sync(0xFFFFFFFFu, na, off));
+                nb_ = fmaxf(nb_, __shfl_xor_sync(0xFFFFFFFFu, nb_, off));
+            }
+            // position 0 is visible to every row, so the maxima are finite from the first tile on
+            const float ca = exp2f(ma - na), cb = exp2f(mb - nb_);
+            ma = na;
+            mb = nb_;
+            la *= ca;
+            lb *= cb;
+#pragma unroll
+            for (int i = 0; i < HD / 8; ++i) {
+                o[i][0] *= ca;
+                o[i][1] *= ca;
+                o[i][2] *= cb;
+                o[i][3] *= cb;
+            }
+#pragma unroll
+            for (int kk = 0; kk < kPaTile / 16; ++kk) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float* e = s[2 * kk + h];
+                    e[0] = exp2f(e[0] - ma);
+                    e[1] = exp2f(e[1] - ma);
+                    e[2] = exp2f(e[2] - mb);
+                    e[3] = exp2f(e[3] - mb);
+                    la += e[0] + e[1];
+                    lb += e[2] + e[3];
+                    __half hh[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        hh[c] = __float2half_rn(e[c]);
+                        e[c] -= __half2float(hh[c]);
+                    }
+                    hi[2 * h] = pa_pack(hh[0], hh[1]);
+                    hi[2 * h + 1] = pa_pack(hh[2], hh[3]);
+                    lo[2 * h] = pa_pack(__float2half_rn(e[0]), __float2half_rn(e[1]));
+                    lo[2 * h + 1] = pa_pack(__float2half_rn(e[2]), __float2half_rn(e[3]));
+                }
+#pragma unroll
+                for (int nb = 0; nb < HD / 16; ++nb) {
+                    const int r = kk * 16 + (lane & 15), c = 2 * nb + (lane >> 4);
+                    uint32_t b[4];
+                    pa_ldsm4_t(b, vb + r * kRowBytes + ((c ^ (r & 7)) << 4));
+                    pa_mma(o[2 * nb], hi, b[0], b[1]);
+                    pa_mma(o[2 * nb + 1], hi, b[2], b[3]);
+                    pa_mma(o[2 * nb], lo, b[0], b[1]);
+                    pa_mma(o[2 * nb + 1], lo, b[2], b[3]);
+                }
+            }
+        }
+        __syncthreads();  // the tile's buffer is free for the load after next
+    }
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+        la += __shfl_xor_sync(0xFFFFFFFFu, la, off);
+        lb += __shfl_xor_sync(0xFFFFFFFFu, lb, off);
+    }
+    const float ia = 1.0f / la, ib = 1.0f / lb;
+    const int ra = tok0 + g, rb = tok0 + g + 8;
+#pragma unroll
+    for (int i = 0; i < HD / 8; ++i) {
+        const int d = i * 8 + 2 * t4;
+        if (ra < T)
+            *reinterpret_cast<__half2*>(out + (static_cast<size_t>(ra) * num_heads + head) * HD + d) =
+                __halves2half2(__float2half_rn(o[i][0] * ia), __float2half_rn(o[i][1] * ia));
+        if (rb < T)
+            *reinterpret_cast<__half2*>(out + (static_cast<size_t>(rb) * num_heads + head) * HD + d) =
+                __halves2half2(__float2half_rn(o[i][2] * ib), __float2half_rn(o[i][3] * ib));
+    }
+}
+
+}  // namespace
+
+bool prefill_attention_supported(int num_heads, int num_kv_heads, int head_dim) {
+    return num_kv_heads > 0 && num_heads % num_kv_heads == 0 && num_heads / num_kv_heads <= 8 &&
+           (head_dim == 64 || head_dim == 128);
+}
+
+// Q and out: T rows of num_heads * head_dim half, 16-byte aligned caches (num_kv_heads, max_seq_len, head_dim) half
+int prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads, int num_kv_heads,
+                      int head_dim, int max_seq_len, float scale, const int* d_pos, void* stream) {
+    const int G = num_heads / num_kv_heads;
+    const int R = max(1, 4 / G);  // at least four warps share a K / V tile
+    const float scale_log2 = scale * 1.44269504088896340736f;
+    const size_t smem = 4 * static_cast<size_t>(kPaTile) * head_dim * 2;
+    auto kernel = head_dim == 64 ? prefill_attention_kernel<64> : prefill_attention_kernel<128>;
+    if (int rc = ensure_dynamic_smem("prefill_attention", kernel, smem)) return rc;
+    return launch("prefill_attention", kernel, dim3((T + R * kPaRows - 1) / (R * kPaRows), num_kv_heads), dim3(32 * G * R),
+                  smem, stream, static_cast<const __half*>(Q), static_cast<const __half*>(K), static_cast<const __half*>(V),
+                  static_cast<__half*>(out), T, num_heads, G, R, max_seq_len, scale_log2, d_pos);
+}
+
+}  // namespace spb

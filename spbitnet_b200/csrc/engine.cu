@@ -493,8 +493,12 @@ int enqueue_prefill_chunk(spb_engine* e, int T, bool last) {
         }
         if ((rc = rope_scatter(e->pf_q, e->pf_k, e->pf_v, kc, vc, nh, nkv, hd, c.max_position_embeddings,
                                c.rope_theta, e->d_pos, s, T))) return rc;
-        if ((rc = decode_attention_pos(e->pf_q, kc, vc, e->pf_attn, nh, nkv, hd, c.max_position_embeddings,
-                                       attn_scale, e->d_pos, s, T))) return rc;
+        rc = prefill_attention_supported(nh, nkv, hd)
+                 ? prefill_attention(e->pf_q, kc, vc, e->pf_attn, T, nh, nkv, hd, c.max_position_embeddings, attn_scale,
+                                     e->d_pos, s)
+                 : decode_attention_pos(e->pf_q, kc, vc, e->pf_attn, nh, nkv, hd, c.max_position_embeddings, attn_scale,
+                                        e->d_pos, s, T);
+        if (rc) return rc;
         if ((rc = absmax_quantize_rows(e->pf_attn, e->pf_xq, am1, nh * hd, T, s))) return rc;
         if ((rc = prefill_linear(e, L.lin[3], am1, e->pf_o, T, e->stream, e->pf_acc))) return rc;
         if ((rc = residual_norm_quant(e->pf_o, L.norm[2], e->pf_x, L.norm[1], nullptr, e->pf_xq, am0, H,

@@ -40,6 +40,11 @@ int rope_scatter(void* q, const void* k, const void* v, void* kcache, void* vcac
 int decode_attention_pos(const void* Q, const void* K, const void* V, void* out, int num_heads,
                          int num_kv_heads, int head_dim, int max_seq_len, float scale, const int* d_pos,
                          void* stream, int vectors = 1, size_t seq_stride = 0);
+// attention_prefill.cu: causal attention of T tokens at positions *d_pos .. over the caches, on the tensor cores; takes
+// whole GQA groups of up to 8 heads and head dims 64 and 128
+int prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads, int num_kv_heads,
+                      int head_dim, int max_seq_len, float scale, const int* d_pos, void* stream);
+bool prefill_attention_supported(int num_heads, int num_kv_heads, int head_dim);
 // attention.cu: split-KV decode attention.  seq_len comes from *d_pos + 1 when d_pos is given.
 // `counters` (optional): num_kv_heads zeroed words; with them the merge of a KV head's chunks runs inside the same
 // launch, in the block that finishes last, instead of as a second kernel.  They are left at zero.
