@@ -135,11 +135,11 @@ int spb_sparse_bitlinear_gemm(const uint32_t* meta, const uint32_t* values, cons
                               const float* d_absmax, float gamma, int32_t* acc_workspace, int rows, int cols,
                               int n, int meta_row_stride, int values_row_stride, void* stream);
 
-/* Which form spb_sparse_ternary_gemm uses: 0 (default) = automatic: up to 32 batch rows the warp-level
- * sparse MMA form (mma.sp m16n8k64, operands re-encoded in registers; needs cols % 256 == 0, row strides
- * that are multiples of 4 words and 16-byte aligned meta / values / X), above that the tcgen05 sparse form
- * (tcgen05.mma.sp: sign bytes as the compressed operand, index pairs in tensor memory), the SIMT form where
- * the layout allows neither; 1 = SIMT form, 3 = tcgen05 sparse form for any n, 4 = warp-level sparse MMA
+/* Which form spb_sparse_ternary_gemm uses: 0 (default) = automatic: up to 8 batch rows of matrices up to 40 M weights the
+ * warp-level sparse MMA form (mma.sp m16n8k64, operands re-encoded in registers; needs cols % 256 == 0, row strides
+ * that are multiples of 4 words and 16-byte aligned meta / values / X), else the tcgen05 sparse form
+ * (tcgen05.mma.sp: sign bytes as the compressed operand, index pairs in tensor memory), which takes any layout;
+ * 1 = SIMT form, 3 = tcgen05 sparse form for any n, 4 = warp-level sparse MMA
  * form where it applies.  Other values behave like 0.  Results are identical.  Returns the previous setting. */
 int spb_set_gemm_variant(int variant);
 /* Weight rows per block of the tcgen05 sparse form: 0 (default) = automatic, 1 = 128 rows, 2 = 256 rows (two

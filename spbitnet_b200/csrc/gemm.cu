@@ -7,6 +7,7 @@
 // into 32 packed int8x4 weight words held in registers and replays them against
 // kBatchTile activation rows staged in shared memory, so the weight stream is read
 // from HBM once per kBatchTile rows.
+#include "gemm_tcsp_ws.cuh"
 #include "spb_common.cuh"
 
 namespace spb {
@@ -141,8 +142,6 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_generic_kernel(const GemmAr
     if (lane == 0) a.Y[static_cast<size_t>(j) * a.rows + row] = acc;
 }
 
-int gemm_tcsp_ws_launch(const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y, int rows, int cols,
-                        int n, int meta_stride, int values_stride, void* stream, const GemmEpilogue* ep);
 // prefill.cu
 int dequantize_rows(const int32_t* acc, void* out, const float* d_absmax, float gamma, int rows, int vectors,
                     void* stream);
@@ -151,11 +150,13 @@ bool gemm_mmasp_supported(const uint32_t* meta, const uint32_t* values, const in
 int gemm_mmasp_launch(const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y, int rows, int cols,
                       int n, int meta_stride, int values_stride, void* stream, const GemmEpilogue* ep);
 
-// 0 automatic (up to 32 batch rows: warp-level sparse MMA form; above: tcgen05 sparse form; SIMT where the layout
-// allows neither), 1 SIMT form, 3 tcgen05 sparse form, 4 warp-level sparse MMA form (3 and 4 whenever the layout
-// allows)
+// 0 automatic, 1 SIMT form, 3 tcgen05 sparse form, 4 warp-level sparse MMA form where the layout allows it, else 3.
+// Automatic: the warp-level form costs one pass of re-encoding per eight batch rows and starts sooner, so it keeps up to
+// eight rows (6912x2560, n = 8: 4.4 against 6.3 us; n = 16: 6.8 against 6.3; n = 64: 14.9 against 7.0) of matrices up to
+// 40 M weights (8192x8192, n = 8: 12.8 against 11.1 us); the tcgen05 form takes the rest and every layout.
 static int g_gemm_variant = 0;
-constexpr int kMmaSpAutoMaxN = 32;
+constexpr int kMmaSpAutoMaxN = 8;
+constexpr long long kMmaSpAutoMaxWeights = 40ll << 20;
 
 }  // namespace spb
 
@@ -209,16 +210,17 @@ static int gemm_dispatch(const char* name, const uint32_t* meta, const uint32_t*
     auto al = [](const void* p, size_t k) { return (reinterpret_cast<uintptr_t>(p) & (k - 1)) == 0; };
     const bool fast = cols % 128 == 0 && cols / 128 <= 512 && meta_row_stride % 4 == 0 &&
                       values_row_stride % 2 == 0 && al(meta, 16) && al(values, 8) && al(X, 16);
-    // up to 32 batch rows the warp-level form always wins; up to 64 it still does when the tcgen05 form, with
-    // its tiles of 128 weight rows, would leave most SMs idle (measured at 2560x6912: 18.8 against 30.1 us)
-    const int mma_auto_max_n = (rows + 127) / 128 < sm_count() / 4 ? 64 : kMmaSpAutoMaxN;
+    const int mma_auto_max_n = static_cast<long long>(rows) * cols <= kMmaSpAutoMaxWeights ? kMmaSpAutoMaxN : 0;
     if ((g_gemm_variant == 0 || g_gemm_variant == 4) &&
         gemm_mmasp_supported(meta, values, X, rows, cols, n, meta_row_stride, values_row_stride,
                              g_gemm_variant == 4 ? 4096 : mma_auto_max_n))
         return gemm_mmasp_launch(meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream, ep);
-    if (fast && g_gemm_variant != 1) {  // warp-specialised tcgen05 sparse form
-        const int rc = gemm_tcsp_ws_launch(meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream, ep);
-        if (rc != SPB_E_UNSUPPORTED) return rc;  // no tensor map of X on this system: the SIMT form below
+    if (g_gemm_variant != 1 && (fast || !ep || Y)) {
+        // tcgen05 sparse form, any layout.  The scaled output of a layout without 16-byte rows keeps asking for the workspace
+        // that spb_sparse_bitlinear_gemm documents, although this form does not write to it.
+        const TcspMat m{meta, values, ep ? static_cast<void*>(ep->out) : Y, ep ? ep->gamma : 0.0f, rows, meta_row_stride,
+                        values_row_stride};
+        return gemm_tcsp_ws_launch(&m, 1, X, ep ? ep->absmax : nullptr, cols, n, stream);
     }
     if (ep) {  // the SIMT forms write int32 sums: run them into the workspace, then scale row by row
         if (!Y) return fail(SPB_E_UNSUPPORTED, "%s: this layout needs acc_workspace (n * rows int32)", name);
@@ -229,6 +231,23 @@ static int gemm_dispatch(const char* name, const uint32_t* meta, const uint32_t*
     }
     return gemm_dispatch_int(name, meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream, fast);
 }
+
+namespace spb {
+
+// BitLinear layers of one width on the same n quantised rows: one launch where the tcgen05 form takes them all (a matrix of
+// five row tiles has no SMs to fill on its own), else one after the other.
+int bitlinear_gemm_group(const TcspMat* mats, int nmat, const int8_t* Xq, const float* absmax, int cols, int n,
+                         int32_t* acc_workspace, void* stream) {
+    const bool one = nmat <= kWsMaxMats && (g_gemm_variant == 3 || (g_gemm_variant == 0 && n > kMmaSpAutoMaxN)) && cols % 4 == 0;
+    if (one) return gemm_tcsp_ws_launch(mats, nmat, Xq, absmax, cols, n, stream);
+    for (int i = 0; i < nmat; ++i)
+        if (int rc = spb_sparse_bitlinear_gemm(mats[i].meta, mats[i].values, Xq, mats[i].out, absmax, mats[i].gamma, acc_workspace,
+                                               mats[i].rows, cols, n, mats[i].meta_stride, mats[i].values_stride, stream))
+            return rc;
+    return SPB_OK;
+}
+
+}  // namespace spb
 
 // The SIMT forms (no fused epilogue).
 static int gemm_dispatch_int(const char* name, const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y,

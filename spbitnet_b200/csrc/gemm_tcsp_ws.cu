@@ -1,60 +1,82 @@
-// Batched sparse-ternary product on tcgen05.mma.sp, warp-specialised form (sm_100a).
+// Batched sparse-ternary product on tcgen05.mma.sp, warp-specialised (sm_100a).
 //
 //   Y[j, r] = sum_c W[r, c] * X[j, c]      W: rows x cols compressed 2:4 ternary, X: n x cols int8
 //
 // Operands: the sign bytes (+1 / -1) of a tile as the compressed A operand in shared memory (K-major, 128-byte
-// swizzle), the index pairs as metadata in tensor memory (one byte per 8 columns, lane = weight row), the
-// activation tiles by tensor-map bulk copies, int32 accumulators in tensor memory.  A first form in which one
-// thread issued the copies and the MMAs between two block-wide barriers per step cost about 2450 cycles per
-// step of which the re-encoding was 500 (the rest: that thread's serial chain with 255 threads parked).  Here
-// the block has three roles that only meet at mbarriers:
-//   warps 0-7 and 12-19      re-encode, as two groups of 256 threads that take alternate steps: wait for a
-//                            free stage, write the A tile and the metadata of a step, arrive on the
-//                            stage's "a_full" barrier;
-//   warp 8     (one lane)    issues the MMAs: waits for a_full and b_full of a stage, issues four
-//                            tcgen05.mma.sp, commits to the stage's "free" barrier;
-//   warp 9     (one lane)    feeds the activations: waits for a free stage, expect_tx + two tensor-map
-//                            bulk copies onto the stage's "b_full" barrier.
-// So the re-encoding of step k + 1 runs under the MMAs of step k, and nobody waits at a block barrier
-// inside the loop.  The epilogue (tcgen05.ld, stores) is done by the re-encoding warps after the last commit.
-// Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run
-// out of their own bounds, the copy warp waits (bounded) for its copies in flight, tensor memory is freed
-// and the block returns.
+// swizzle), the index pairs as metadata in tensor memory (one byte per 8 columns, lane = weight row), the activation
+// tiles by tensor-map bulk copies, int32 accumulators in tensor memory.  A block owns 128 weight rows (mh = 1) or 256
+// (mh = 2, two accumulators on one activation tile), up to 256 (240) batch rows and a range of K; its roles meet only at
+// mbarriers:
+//   warps 0-15  re-encode: the packed words of a step (256 columns) from shared memory to sign bytes and index pairs.
+//               mh = 1: two groups of eight warps take alternate steps; mh = 2: group g takes rows 128 g .. of every step;
+//   warp 16     issues the MMAs (one lane), half a step at a time;
+//   warp 17     brings the activation tiles: one tensor-map copy per half step (128 columns);
+//   warp 18     brings the packed weights: tensor-map copies of 512 columns of every row, as they lie in memory, several
+//               chunks ahead.  They depend on no predecessor and start before the dependency wait.
+// With few row tiles the K extent is cut over a cluster of S blocks, each of which adds and stores a slice of the columns
+// from all blocks' partial sums (distributed shared memory).  Sums are integers: same bits.
+//
+// What bounds it.  An MMA of 64 columns takes 47 + N / 2 clocks.  With wide batches the tensor pipe and the activation
+// traffic out of L2 (256-row blocks halve it); with few batch rows the re-encoding, 650 clocks per step; below a dozen
+// steps per block the start of a block (2 us) and, with a split, the exchange at 13 B per clock and SM.
+//   28672 x 8192, n = 1024: 275 -> 129 us;  n = 64: 105 -> 23 us;  2560 x 6912, n = 200: 20.1 -> 9.7 us, against a form in
+//   which weights came by 16-byte loads of a row per lane (32 cache lines per instruction), signs through a table in shared
+//   memory, and the MMA thread divided four times per half step to find its ring slots (1050 of 1100 clocks).
+// A sign word of 32 weights becomes 32 bytes by a bit transpose and eight byte permutes whose selectors are the sign bits
+// themselves: 21 instructions, no table.
+//
+// LAYOUT = kTiled: cols % 16 == 0, row strides multiples of 4 words, 16-byte aligned meta / values / X (tensor maps).
+// LAYOUT = kAny: any other: the re-encoding warps load their words themselves, eight warps copy the activation tiles.
+//
+// Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run out of their own
+// bounds, the copy warps wait (bounded) for their copies in flight, tensor memory is freed and the block returns.
 #include <cuda.h>
 
+#include <cmath>
 #include <cstring>
 
-#include "spb_common.cuh"
+#include "gemm_tcsp_ws.cuh"
 
 namespace spb {
 
-constexpr int kWsExpanders = 256;
-// warps 0-7: re-encoding group 0 (even steps); 8: MMA; 9: copy; 10-11: idle (a warp may only touch the tensor-memory
-// lanes 32 * (warp % 4) .. + 31, so the second group starts at a multiple of four); 12-19: re-encoding group 1 (odd steps)
-constexpr int kWsGroup1Warp = 12;
-constexpr int kWsThreads = 32 * (kWsGroup1Warp + 8);
 constexpr int kWsTileM = 128;
 constexpr int kWsStepK = 256;                  // logical columns per step: two units per row
-constexpr int kWsABytes = kWsTileM * 128;      // compressed A tile: 128 rows x 128 bytes
-constexpr int kWsMaxStages = 4;
-constexpr int kWsSignLutBytes = 16 * 32 * 4;
+constexpr int kWsABytes = kWsTileM * 128;      // compressed A tile of a step: 128 rows x 128 bytes
+constexpr int kWsWBytes = kWsTileM * (64 + 32);  // packed words of 512 columns of 128 rows: meta, values
+constexpr int kWsExpandWarps = 16;
+constexpr int kWsMmaWarp = 16, kWsXWarp = 17, kWsWWarp = 18;
+constexpr int kWsThreadsTiled = 32 * 19;
+constexpr int kWsCopyWarps = 8;                // kAny: warps 17 .. 24 copy the activation tiles
+constexpr int kWsThreadsAny = 32 * (kWsXWarp + kWsCopyWarps);
+constexpr int kWsMaxRing = 8;
+constexpr int kWsBarBytes = 512, kWsScaleBytes = 1024;
 constexpr long long kWsWaitCycles = 40000000;
+constexpr int kWsSmemCap = 226 * 1024;
 
-struct WsArgs {
+enum WsLayout { kTiled = 0, kAny = 1 };
+
+struct WsMat {
     const uint32_t* meta;
     const uint32_t* values;
-    int32_t* Y;
-    int rows, cols, n;
-    int meta_stride, values_stride;
-    int nt;         // batch rows per block: multiple of 16, at most 256
-    int stages;     // ring depth (2..kWsMaxStages)
-    int tmem_cols;  // power of two >= nt + 8 * stages
-    int groups;     // re-encoding groups in use: 2 (alternate steps), or 1 (warps 12-19 idle)
-    int mh;         // weight-row halves per block: 1 (128 rows), or 2 (256 rows: group g re-encodes rows 128 g .. of every
-                    // step, both halves multiply the same activation tile into their own accumulator)
-    GemmEpilogue ep;  // ep.out set: scaled half output instead of Y
-    int* timeouts;        // counter of waits that ran out (pinned host memory, system-scope atomics), may be null
+    void* out;  // int32 sums or half
+    float gamma;
+    int rows, meta_stride, values_stride, tile0;  // tile0: first row tile of this matrix in the grid
+};
+struct WsArgs {
+    WsMat m[kWsMaxMats];
+    const int8_t* X;
+    const float* absmax;
+    int nmat, cols, n;
+    int nt;                 // batch rows per block: multiple of 16, at most 256
+    int mh;                 // 128-row halves per block
+    int sa, sb, sw;         // ring depths: A (steps), activations (half steps), packed words (512 columns)
+    int tmem_cols;          // power of two >= mh * (nt + 8 * sa)
+    int split;              // blocks per cluster that share the K extent
+    int* timeouts;          // counter of waits that ran out (pinned host memory, system-scope atomics), may be null
     long long wait_cycles;  // bound of every wait in the kernel
+};
+struct WsMaps {
+    CUtensorMap x, meta[kWsMaxMats], values[kWsMaxMats];
 };
 
 // 0 automatic, 1 / 2 force one / two weight-row halves per block (spb_set_gemm_row_halves; testing and measurement)
@@ -83,9 +105,17 @@ __device__ __forceinline__ uint32_t ws_idesc(int m, int n) {
 }
 // Bounded by time, not by polls (a poll may suspend for a while): kWsWaitCycles is about 20 ms at 2 GHz.
 __device__ __forceinline__ bool ws_wait(uint32_t mbar, uint32_t parity, long long limit) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (done) return true;
     const long long t0 = clock64();
     for (;;) {
-        uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -97,8 +127,68 @@ __device__ __forceinline__ bool ws_wait(uint32_t mbar, uint32_t parity, long lon
         if (clock64() - t0 > limit) return false;
     }
 }
+__device__ __forceinline__ void ws_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void ws_init(uint32_t mbar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
+}
+__device__ __forceinline__ void ws_expect(uint32_t mbar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ws_tma(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
+}
+__device__ __forceinline__ void ws_commit(uint32_t mbar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+// Position in a ring of barriers: stage and phase, advanced without a division.
+struct WsCursor {
+    int s = 0;
+    uint32_t ph = 0;
+    __device__ __forceinline__ void advance(int depth, int by = 1) {
+        s += by;
+        if (s >= depth) {
+            s -= depth;
+            ph ^= 1u;
+        }
+    }
+};
+__device__ __forceinline__ bool ws_elect() {
+    uint32_t e;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(e));
+    return e != 0;
+}
+// One MMA: 128 rows x N, 64 logical columns.  a_lo, b_lo: low words of the operands' descriptors.
+__device__ __forceinline__ void ws_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t meta) {
+    constexpr uint32_t hi = (1024u >> 4) | (1u << 14) | (1u << 30);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 a, {%1, %6};\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "tcgen05.mma.sp.cta_group::1.kind::i8 [%0], a, b, [%5], %3, p;\n\t}"
+        :
+        : "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(meta), "r"(hi)
+        : "memory");
+}
+// 16-byte piece c of row r of a 128-byte-swizzled tile
 __device__ __forceinline__ uint32_t ws_swz(int r, int c) {
     return static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
+}
+// Bitmaps of zero (past the end of a row or of the matrix: the activations there are zero, the rows are not stored)
+// become {0, 1}: the tensor core is only given valid pairs.
+__device__ __forceinline__ uint32_t ws_fill_empty(uint32_t m) {
+    const uint32_t h = m | (m >> 1);
+    const uint32_t z = ~(h | (h >> 2)) & 0x11111111u;
+    return m | z | (z << 1);
 }
 // Eight bitmaps (two of four bits set each) -> eight index pairs {low index | high index << 2}.
 __device__ __forceinline__ uint32_t ws_index_pairs(uint32_t m) {
@@ -107,46 +197,80 @@ __device__ __forceinline__ uint32_t ws_index_pairs(uint32_t m) {
     const uint32_t t2 = (0x22222222u & (~ml & ~m)) | (~0x22222222u & (m | ml));
     return (t1 & 0x55555555u) | (t2 & 0xAAAAAAAAu);
 }
+// 32 sign bits -> 32 bytes of +1 / -1 in order.  Transposing the 4 x 4 bits of each 16-bit half puts the signs 4 r .. 4 r
+// + 3 at bit r of the half's four nibbles; a byte permute with the nibbles as selectors and a source whose byte i is -1
+// where bit r of i is set then yields those four bytes.  A selector's top bit means "replicate the sign", so the nibbles
+// are masked to three bits and bit 3 is read at bit 2.
+__device__ __forceinline__ void ws_sign_bytes(uint32_t v, uint32_t (&w)[8]) {
+    uint32_t t = (v ^ (v >> 3)) & 0x0A0A0A0Au;
+    v ^= t ^ (t << 3);
+    t = (v ^ (v >> 6)) & 0x00CC00CCu;
+    v ^= t ^ (t << 6);
+    const uint32_t lo = v & 0x77777777u, hi = (v >> 1) & 0x44444444u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t l = h ? lo >> 16 : lo, u = h ? hi >> 16 : hi;
+        w[4 * h + 0] = __byte_perm(0xFF01FF01u, 0xFF01FF01u, l);
+        w[4 * h + 1] = __byte_perm(0xFFFF0101u, 0xFFFF0101u, l);
+        w[4 * h + 2] = __byte_perm(0x01010101u, 0xFFFFFFFFu, l);
+        w[4 * h + 3] = __byte_perm(0x01010101u, 0xFFFFFFFFu, u);
+    }
+}
 
-// HALF_OUT: the epilogue writes the scaled half output (a.ep) instead of the int32 sums
-template <bool HALF_OUT>
-__global__ void __launch_bounds__(kWsThreads, 1) gemm_tcsp_ws_kernel(const WsArgs a, const __grid_constant__ CUtensorMap tmap_x) {
+template <bool HALF_OUT, int LAYOUT>
+__global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThreadsAny, 1)
+    gemm_tcsp_ws_kernel(const WsArgs a, const __grid_constant__ WsMaps maps) {
     extern __shared__ uint8_t ws_raw[];
-    // [sign table 2 KB][barriers + tmem slot 128 B] ... 1024-aligned: [stage: A 16 KB x mh | B0 nt*128 | B1 nt*128] x stages
-    uint32_t* sgn = reinterpret_cast<uint32_t*>(ws_raw);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(ws_raw + kWsSignLutBytes);
-    uint64_t* a_full = bars;                      // [stage]: 256 arrivals, the re-encoded tile and its metadata are written
-    uint64_t* b_full = bars + kWsMaxStages;       // [stage]: the two activation tiles have landed
-    uint64_t* free_b = bars + 2 * kWsMaxStages;   // [stage]: the MMAs that read the stage are done
-    uint64_t* done_b = bars + 3 * kWsMaxStages;   // all MMAs of the block are done
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ws_raw + kWsSignLutBytes + 112);
+    // [barriers][row scales] ... 1024-aligned: [A ring][activation ring][packed-word ring]; the epilogue's sums take the
+    // place of the rings when the products are done
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ws_raw);
     const uint32_t raw_s = ws_smem(ws_raw);
-    const uint32_t stage0_s = (raw_s + kWsSignLutBytes + 128 + 1023) & ~1023u;
-    uint8_t* stage0 = ws_raw + (stage0_s - raw_s);
-    const int b_bytes = a.nt * 128;  // one of the two activation sub-tiles
-    const int a_bytes = a.mh * kWsABytes;
-    const int stage_bytes = a_bytes + 2 * b_bytes;
-    const int S = a.stages;
+    const uint32_t a_full = raw_s, a_free = raw_s + 64, b_full = raw_s + 128, b_free = raw_s + 192, w_full = raw_s + 256,
+                   w_free = raw_s + 320, done_b = raw_s + 384;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 50);
+    float* scales = reinterpret_cast<float*>(ws_raw + kWsBarBytes);
+    const uint32_t ring_s = (raw_s + kWsBarBytes + kWsScaleBytes + 1023) & ~1023u;
+    const int a_bytes = a.mh * kWsABytes, b_bytes = a.nt * 128, w_bytes = a.mh * kWsWBytes;
+    const uint32_t bring_s = ring_s + a.sa * a_bytes, wring_s = bring_s + a.sb * b_bytes;
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
-    const int row0 = blockIdx.x * kWsTileM * a.mh;
+    int mi = 0;
+    if (a.nmat > 1 && static_cast<int>(blockIdx.x) >= a.m[1].tile0) mi = 1;
+    if (a.nmat > 2 && static_cast<int>(blockIdx.x) >= a.m[2].tile0) mi = 2;
+    const WsMat m = mi == 0 ? a.m[0] : mi == 1 ? a.m[1] : a.m[2];
+    const int row0 = (static_cast<int>(blockIdx.x) - m.tile0) * kWsTileM * a.mh;
     const int n0 = blockIdx.y * a.nt;
-    const int upr = a.cols >> 7;
-    const int nsteps = (upr + 1) >> 1;
+    const int all_steps = (a.cols + kWsStepK - 1) / kWsStepK;
+    const int s0 = static_cast<int>(blockIdx.z) * all_steps / a.split;
+    const int nsteps = (static_cast<int>(blockIdx.z) + 1) * all_steps / a.split - s0;
 
     grid_dep_launch();
-    for (int i = tid; i < 16 * 32; i += kWsThreads) {  // byte b of an entry = -1 if bit b of the nibble is set, else +1
-        const uint32_t t = ((static_cast<uint32_t>(i) >> 5) * 0x00204081u) & 0x01010101u;
-        sgn[i] = (t * 0xFEu) | 0x01010101u;
-    }
-    if (tid == 0) {
-        for (int s = 0; s < kWsMaxStages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ws_smem(a_full + s)), "r"(kWsExpanders * a.mh));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ws_smem(b_full + s)));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ws_smem(free_b + s)));
+    const int nchunks = (nsteps + 1) >> 1;
+    auto load_chunk = [&](int c, int s) {  // packed words of 512 columns: 16 words of meta and 8 of values per row
+        const uint32_t bar = w_full + 8 * s, dst = wring_s + s * w_bytes;
+        const int k2 = s0 + 2 * c;
+        ws_expect(bar, w_bytes);
+        ws_tma(dst, &maps.meta[mi], 8 * k2, row0, bar);
+        ws_tma(dst + a.mh * kWsTileM * 64, &maps.values[mi], 4 * k2, row0, bar);
+    };
+    if (LAYOUT == kTiled && tid == 32 * kWsWWarp) {  // the first chunks leave before the block has set itself up (1100 clocks)
+        for (int s = 0; s < a.sw; ++s) {
+            ws_init(w_full + 8 * s, 1);
+            ws_init(w_free + 8 * s, kWsExpandWarps);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ws_smem(done_b)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int s = 0; s < min(a.sw, nchunks); ++s) load_chunk(s, s);
+    }
+    if (tid == 32 * kWsXWarp) {
+        if (LAYOUT == kTiled) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
+        for (int s = 0; s < kWsMaxRing; ++s) {
+            ws_init(a_full + 8 * s, 8 * a.mh);
+            ws_init(a_free + 8 * s, 1);
+            ws_init(b_full + 8 * s, LAYOUT == kTiled ? 1 : kWsCopyWarps);
+            ws_init(b_free + 8 * s, 1);
+        }
+        ws_init(done_b, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -162,195 +286,306 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_tcsp_ws_kernel(const WsArg
     const uint32_t tmem_e = tmem_d + static_cast<uint32_t>(a.nt * a.mh);  // metadata slots behind the accumulators
     bool ok = true;
 
-    if (warp == 9) {
-        // ---- copy warp: activation tiles of every step, as soon as their stage is free ----------------------
+    if (LAYOUT == kTiled && warp == kWsWWarp) {
+        // ---- packed weights: 512 columns of every row per chunk ---------------------------------------------------
+        if (lane == 0) {
+            WsCursor w;
+            int issued = min(a.sw, nchunks);
+            w.ph = 1;
+            for (; issued < nchunks; ++issued, w.advance(a.sw)) {
+                if (!(ok = ws_wait(w_free + 8 * w.s, w.ph ^ 1u, a.wait_cycles))) break;
+                load_chunk(issued, w.s);
+            }
+            for (int c = max(0, issued - a.sw); c < issued; ++c)  // nothing in flight when the block leaves
+                if (!ws_wait(w_full + 8 * (c % a.sw), static_cast<uint32_t>(c / a.sw) & 1u, a.wait_cycles)) ok = false;
+            if (!ok) ws_count_timeout(a.timeouts);
+        }
+    } else if (LAYOUT == kTiled && warp == kWsXWarp) {
+        // ---- activation tiles ----------------------------------------------------------------------------------------
         if (lane == 0) {
             grid_dep_wait();  // X may be a predecessor's output
+            WsCursor x;
             int issued = 0;
-            for (int kc = 0; kc < nsteps && ok; ++kc) {
-                const int s = kc % S;
-                if (kc >= S) ok = ws_wait(ws_smem(free_b + s), static_cast<uint32_t>(kc / S - 1) & 1u, a.wait_cycles);
-                if (!ok) break;
-                const uint32_t fb = ws_smem(b_full + s);
-                uint8_t* sb = stage0 + static_cast<size_t>(s) * stage_bytes + a_bytes;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
-                             "r"(static_cast<uint32_t>(2 * b_bytes))
-                             : "memory");
-#pragma unroll
-                for (int h = 0; h < 2; ++h)  // columns [256 kc + 128 h, +128) of batch rows [n0, n0 + nt)
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                            ws_smem(sb + h * b_bytes)),
-                        "l"(reinterpret_cast<uint64_t>(&tmap_x)), "r"(kc * kWsStepK + 128 * h), "r"(n0), "r"(fb)
-                        : "memory");
-                issued = kc + 1;
+            for (; issued < 2 * nsteps; ++issued, x.advance(a.sb)) {
+                if (!(ok = ws_wait(b_free + 8 * x.s, x.ph ^ 1u, a.wait_cycles))) break;
+                ws_expect(b_full + 8 * x.s, b_bytes);
+                ws_tma(bring_s + x.s * b_bytes, &maps.x, s0 * kWsStepK + issued * 128, n0, b_full + 8 * x.s);
             }
-            // nothing of this block's copies may be in flight when it leaves: the last S issued steps
-            for (int kc = max(0, issued - S); kc < issued; ++kc)
-                if (!ws_wait(ws_smem(b_full + kc % S), static_cast<uint32_t>(kc / S) & 1u, a.wait_cycles)) ok = false;
+            for (int h = max(0, issued - a.sb); h < issued; ++h)
+                if (!ws_wait(b_full + 8 * (h % a.sb), static_cast<uint32_t>(h / a.sb) & 1u, a.wait_cycles)) ok = false;
             if (!ok) ws_count_timeout(a.timeouts);
         }
-    } else if (warp == 8) {
-        // ---- MMA warp: four tcgen05.mma.sp per step, as soon as both operands of the stage are there ----------
-        if (lane == 0) {
-            const uint32_t idesc = ws_idesc(kWsTileM, a.nt);
-            for (int kc = 0; kc < nsteps; ++kc) {
-                const int s = kc % S;
-                const uint32_t par = static_cast<uint32_t>(kc / S) & 1u;
-                ok = ws_wait(ws_smem(a_full + s), par, a.wait_cycles) && ws_wait(ws_smem(b_full + s), par, a.wait_cycles);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = stage0_s + static_cast<uint32_t>(s) * stage_bytes;
-                const uint64_t db0 = ws_smem_desc(sa + a_bytes), db1 = ws_smem_desc(sa + a_bytes + b_bytes);
-                for (int h = 0; h < a.mh; ++h) {  // each half of the weight rows into its own accumulator
-                    const uint64_t da = ws_smem_desc(sa + static_cast<uint32_t>(h) * kWsABytes);
-                    const uint32_t td = tmem_d + static_cast<uint32_t>(h * a.nt);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {  // 64 logical columns each: 32 B of A, 64 B of X, two metadata columns
-                        const uint32_t acc = (kc > 0 || k > 0) ? 1u : 0u;
-                        const uint64_t db = ((k & 2) ? db1 : db0) + static_cast<uint64_t>(4 * (k & 1));
-                        const uint32_t te = tmem_e + static_cast<uint32_t>((s * a.mh + h) * 8 + 2 * k);
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.sp.cta_group::1.kind::i8 [%0], %1, %2, [%9], %3, {%5, %6, %7, %8}, p;\n\t}"
-                            :
-                            : "r"(td), "l"(da + 2 * k), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u),
-                              "r"(te)
-                            : "memory");
-                    }
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ws_smem(free_b + s))
-                             : "memory");
-                if (kc == nsteps - 1)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ws_smem(done_b))
-                                 : "memory");
-            }
-            if (!ok) ws_count_timeout(a.timeouts);
-        }
-    } else if (warp < 8 || (warp >= kWsGroup1Warp && a.groups == 2)) {
-        // ---- re-encoding warps, two groups of eight that take alternate steps (a step's re-encoding is a chain of
-        //      dependent loads, table reads and stores: two steps in flight hide its latency).  In a group, thread t
-        //      and thread t + 128 share weight row (t & 127) of the tile; per step the first takes the even unit, the
-        //      second the odd unit.  A warp's rows are the tensor-memory lanes it may access.
-        const int grp = warp < 8 ? 0 : 1;
-        const int ewarp = warp < 8 ? warp : warp - kWsGroup1Warp + 8;  // 0..15 over both groups
-        const int etid = (ewarp & 7) * 32 + lane;                        // 0..255 within the group
-        const int trow = etid & (kWsTileM - 1), thalf = etid >> 7;
-        const int mhalf = a.mh == 2 ? grp : 0;  // which 128 rows of the block this group serves
-        const int wrow = row0 + mhalf * kWsTileM + trow;
-        const bool wvalid = wrow < a.rows;
-        auto load_unit = [&](int step, uint4& mm, uint2& vv, bool& valid) {
-            const int u = 2 * step + thalf;
-            valid = wvalid && u < upr;
-            if (valid) {
-                mm = ld_stream_v4(a.meta + static_cast<size_t>(wrow) * a.meta_stride + u * 4);
-                vv = ld_stream_v2(a.values + static_cast<size_t>(wrow) * a.values_stride + u * 2);
-            }
-        };
-        // the weight words of four steps are in flight
-        uint4 m0 = make_uint4(0, 0, 0, 0), m1 = m0, m2 = m0, m3 = m0;
-        uint2 v0 = make_uint2(0, 0), v1 = v0, v2 = v0, v3 = v0;
-        bool u0 = false, u1 = false, u2 = false, u3 = false;
-        const int gs = a.mh == 2 ? 1 : a.groups;  // step stride of a group (with two row halves every group takes every step)
-        const int k_first = a.mh == 2 ? 0 : grp;
-        if (k_first < nsteps) load_unit(k_first, m0, v0, u0);
-        if (k_first + gs < nsteps) load_unit(k_first + gs, m1, v1, u1);
-        if (k_first + 2 * gs < nsteps) load_unit(k_first + 2 * gs, m2, v2, u2);
-        if (k_first + 3 * gs < nsteps) load_unit(k_first + 3 * gs, m3, v3, u3);
-        const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t sgn_s = raw_s + (static_cast<uint32_t>(lane) << 2);
-        for (int kc = k_first; kc < nsteps; kc += gs) {
-            const int s = kc % S;
-            uint4 mn = make_uint4(0, 0, 0, 0);
-            uint2 vn = make_uint2(0, 0);
-            bool nvalid = false;
-            if (kc + 4 * gs < nsteps) load_unit(kc + 4 * gs, mn, vn, nvalid);
-            if (kc >= S) ok = ws_wait(ws_smem(free_b + s), static_cast<uint32_t>(kc / S - 1) & 1u, a.wait_cycles);
-            ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;  // tcgen05.st below is warp-wide
+    } else if (LAYOUT == kAny && warp >= kWsXWarp) {
+        // ---- activation tiles, any alignment: a warp per batch row and half step, four columns per lane ------------
+        grid_dep_wait();
+        const int cw = warp - kWsXWarp;
+        const bool words = (reinterpret_cast<uintptr_t>(a.X) & 3u) == 0;
+        WsCursor xb;
+        for (int h = 0; h < 2 * nsteps; ++h, xb.advance(a.sb)) {
+            const int s = xb.s;
+            ok = ws_wait(b_free + 8 * s, xb.ph ^ 1u, a.wait_cycles);
+            ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
             if (!ok) break;
-            // metadata: index pairs of this unit's 32 groups -> four tensor-memory columns of the row
-            uint32_t e0 = 0x44444444u, e1 = 0x44444444u, e2 = 0x44444444u, e3 = 0x44444444u;
-            if (u0) {
-                e0 = ws_index_pairs(m0.x);
-                e1 = ws_index_pairs(m0.y);
-                e2 = ws_index_pairs(m0.z);
-                e3 = ws_index_pairs(m0.w);
-            }
-            const uint32_t eaddr = tmem_e + lane_base + static_cast<uint32_t>((s * a.mh + mhalf) * 8 + thalf * 4);
-            asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(eaddr), "r"(e0), "r"(e1), "r"(e2),
-                         "r"(e3)
-                         : "memory");
-            // values: sign nibble -> four bytes of +1 / -1; a unit is four 16-byte chunks of the row
-            const uint32_t sa = stage0_s + static_cast<uint32_t>(s) * stage_bytes + static_cast<uint32_t>(mhalf) * kWsABytes;
-            const uint32_t vw[2] = {v0.x, v0.y};
+            const int col = s0 * kWsStepK + h * 128 + lane * 4;
+            for (int r0 = cw; r0 < a.nt; r0 += 8 * kWsCopyWarps) {
+                uint32_t x[8];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t w[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int nibble = 4 * c + q, sh = 4 * (nibble & 7);
-                    const uint32_t word = vw[nibble >> 3];
-                    const uint32_t t = sh >= 7 ? (word >> (sh - 7)) : (word << (7 - sh));  // nibble at bits 7..10
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[q]) : "r"(sgn_s + (t & 0x780u)));
-                    if (!u0) w[q] = 0u;
-                }
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + ws_swz(trow, thalf * 4 + c)), "r"(w[0]),
-                             "r"(w[1]), "r"(w[2]), "r"(w[3])
-                             : "memory");
-            }
-            m0 = m1; v0 = v1; u0 = u1;
-            m1 = m2; v1 = v2; u1 = u2;
-            m2 = m3; v2 = v3; u2 = u3;
-            m3 = mn; v3 = vn; u3 = nvalid;
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ws_smem(a_full + s)) : "memory");
-        }
-        // ---- epilogue: accumulators -> Y -------------------------------------------------------------
-        if (ok) ok = ws_wait(ws_smem(done_b), 0, a.wait_cycles);
-        ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok) {
-            grid_dep_wait();  // Y may still be read by a predecessor
-            // warp w reads TMEM lanes 32 * (w % 4) .. + 31 (weight rows); the warps that serve the same rows share the
-            // columns (all sixteen with one row half, the eight of a group with two)
-            const int quarter = ewarp & 3;
-            const int csel = a.mh == 2 ? ((ewarp >> 2) & 1) : (ewarp >> 2);
-            const int cstep = a.mh == 2 ? 64 : 64 * a.groups;
-            const int row = row0 + mhalf * kWsTileM + quarter * 32 + lane;
-            for (int c0 = csel * 32; c0 < a.nt; c0 += cstep) {
-                uint32_t r[32];
-                const uint32_t taddr = tmem_d + lane_base + static_cast<uint32_t>(mhalf * a.nt + c0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                      "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                      "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < a.rows) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int j = n0 + c0 + i;
-                        if (c0 + i < a.nt && j < a.n) {
-                            const size_t o = static_cast<size_t>(j) * a.rows + row;
-                            if (HALF_OUT)
-                                a.ep.out[o] = __float2half_rn(__fmul_rn(static_cast<float>(static_cast<int32_t>(r[i])),
-                                                                        dequant_scale(a.ep.gamma, a.ep.absmax[j])));
-                            else
-                                a.Y[o] = static_cast<int32_t>(r[i]);
+                for (int i = 0; i < 8; ++i) {
+                    const int j = n0 + r0 + i * kWsCopyWarps;
+                    x[i] = 0;
+                    if (r0 + i * kWsCopyWarps < a.nt && j < a.n && col < a.cols) {
+                        const int8_t* p = a.X + static_cast<size_t>(j) * a.cols + col;
+                        if (words) {
+                            x[i] = __ldg(reinterpret_cast<const uint32_t*>(p));
+                        } else {
+                            for (int b = 0; b < 4; ++b) x[i] |= static_cast<uint32_t>(static_cast<uint8_t>(p[b])) << (8 * b);
                         }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = r0 + i * kWsCopyWarps;
+                    if (r < a.nt)
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(bring_s + s * b_bytes + ws_swz(r, lane >> 2) + 4 * (lane & 3)),
+                                     "r"(x[i])
+                                     : "memory");
+                }
             }
-        } else if (lane == 0) {
-            ws_count_timeout(a.timeouts);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) ws_arrive(b_full + 8 * s);
+        }
+        if (!ok && lane == 0) ws_count_timeout(a.timeouts);
+    } else if (warp == kWsMmaWarp) {
+        // ---- MMAs: two per half step and 128 rows.  One elected lane; addresses and phases advance by additions only: the
+        //      tensor pipe takes 47 + N / 2 clocks per MMA, so the bookkeeping between two of them counts.
+        if (ws_elect()) {
+            const uint32_t idesc = ws_idesc(kWsTileM, a.nt);
+            const uint32_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;
+            const uint32_t a_lo0 = static_cast<uint32_t>(ws_smem_desc(ring_s)), b_lo0 = static_cast<uint32_t>(ws_smem_desc(bring_s));
+            uint32_t a_lo = a_lo0, b_lo = b_lo0, te = tmem_e, acc = 0;
+            uint32_t abar = a_full, bbar = b_full;  // the matching "free" barriers lie 64 bytes on
+            uint32_t aph = 0, bph = 0;
+            auto half = [&](uint32_t h) {
+                if (!ws_wait(bbar, bph, a.wait_cycles)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                ws_mma(tmem_d, a_lo + 4 * h, b_lo, idesc, acc, te + 4 * h);
+                ws_mma(tmem_d, a_lo + 4 * h + 2, b_lo + 4, idesc, 1, te + 4 * h + 2);
+                if (a.mh == 2) {  // the second half of the weight rows into its own accumulator
+                    ws_mma(tmem_d + a.nt, a_lo + (kWsABytes >> 4) + 4 * h, b_lo, idesc, acc, te + 8 + 4 * h);
+                    ws_mma(tmem_d + a.nt, a_lo + (kWsABytes >> 4) + 4 * h + 2, b_lo + 4, idesc, 1, te + 8 + 4 * h + 2);
+                }
+                acc = 1;
+                ws_commit(bbar + 64);
+                b_lo += b_step;
+                bbar += 8;
+                if (bbar == b_full + 8 * a.sb) {
+                    b_lo = b_lo0;
+                    bbar = b_full;
+                    bph ^= 1u;
+                }
+                return true;
+            };
+            for (int kc = 0; kc < nsteps; ++kc) {
+                ok = ws_wait(abar, aph, a.wait_cycles) && half(0) && half(1);
+                if (!ok) break;
+                ws_commit(abar + 64);
+                a_lo += a_step;
+                te += 8 * a.mh;
+                abar += 8;
+                if (abar == a_full + 8 * a.sa) {
+                    a_lo = a_lo0;
+                    te = tmem_e;
+                    abar = a_full;
+                    aph ^= 1u;
+                }
+            }
+            ws_commit(done_b);
+            if (!ok) ws_count_timeout(a.timeouts);
+        }
+    } else if (warp < kWsExpandWarps) {
+        // ---- re-encoding: thread t and thread t + 128 of a group share a weight row, one takes the even unit (128
+        //      columns) of a step, the other the odd one.  A warp's rows are the tensor-memory lanes it may access.
+        const int grp = warp >> 3;
+        const int etid = (warp & 7) * 32 + lane;
+        const int trow = etid & (kWsTileM - 1), thalf = etid >> 7;
+        const int mhalf = a.mh == 2 ? grp : 0;
+        const int first = a.mh == 2 ? 0 : grp, stride = a.mh == 2 ? 1 : 2;
+        const int wr = mhalf * kWsTileM + trow;  // row within the block's packed words
+        const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        const int mwords = (a.cols + 31) >> 5, vwords = (a.cols + 63) >> 6;
+        auto load_words = [&](int i, uint4& mm, uint2& vv) {  // kAny: step i's words, zero past the row's end
+            uint32_t w[6] = {0, 0, 0, 0, 0, 0};
+            if (row0 + wr < m.rows && i < nsteps) {
+                const int u = 2 * (s0 + i) + thalf;
+                const uint32_t* pm = m.meta + static_cast<size_t>(row0 + wr) * m.meta_stride;
+                const uint32_t* pv = m.values + static_cast<size_t>(row0 + wr) * m.values_stride;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (4 * u + q < mwords) w[q] = __ldg(pm + 4 * u + q);
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    if (2 * u + q < vwords) w[4 + q] = __ldg(pv + 2 * u + q);
+            }
+            mm = make_uint4(w[0], w[1], w[2], w[3]);
+            vv = make_uint2(w[4], w[5]);
+        };
+        const bool row_tail = row0 + a.mh * kWsTileM > m.rows;
+        WsCursor ca, cw;
+        ca.s = first;  // fewer steps than stages ahead: first < sa
+        uint4 mm, mn;
+        uint2 vv, vn;
+        if (LAYOUT == kAny) load_words(first, mn, vn);
+        for (int i = first; i < nsteps; i += stride, ca.advance(a.sa, stride)) {
+            if (LAYOUT == kTiled) {
+                const int s = cw.s, x = i & 1;
+                ok = ws_wait(w_full + 8 * s, cw.ph, a.wait_cycles);
+                ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
+                if (!ok) break;
+                const uint32_t pm = wring_s + s * w_bytes + wr * 64 + (((2 * x + thalf) ^ ((wr >> 1) & 3)) << 4);
+                const uint32_t pv = wring_s + s * w_bytes + a.mh * kWsTileM * 64 + wr * 32 + ((x ^ ((wr >> 2) & 1)) << 4) + 8 * thalf;
+                asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(mm.x), "=r"(mm.y), "=r"(mm.z), "=r"(mm.w) : "r"(pm) : "memory");
+                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(vv.x), "=r"(vv.y) : "r"(pv) : "memory");
+            } else {
+                mm = mn;
+                vv = vn;
+                load_words(i + stride, mn, vn);
+            }
+            if (row_tail || (s0 + i + 1) * kWsStepK > a.cols) {
+                mm.x = ws_fill_empty(mm.x);
+                mm.y = ws_fill_empty(mm.y);
+                mm.z = ws_fill_empty(mm.z);
+                mm.w = ws_fill_empty(mm.w);
+            }
+            uint32_t w0[8], w1[8];
+            const uint32_t e0 = ws_index_pairs(mm.x), e1 = ws_index_pairs(mm.y), e2 = ws_index_pairs(mm.z),
+                           e3 = ws_index_pairs(mm.w);
+            ws_sign_bytes(vv.x, w0);
+            ws_sign_bytes(vv.y, w1);
+            const int sA = ca.s;
+            ok = ws_wait(a_free + 8 * sA, ca.ph ^ 1u, a.wait_cycles);
+            ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;  // tcgen05.st below is warp-wide
+            if (!ok) break;
+            const uint32_t eaddr = tmem_e + lane_base + static_cast<uint32_t>((sA * a.mh + mhalf) * 8 + thalf * 4);
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(eaddr), "r"(e0), "r"(e1), "r"(e2),
+                         "r"(e3)
+                         : "memory");
+            const uint32_t sm = ring_s + sA * a_bytes + mhalf * kWsABytes;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t* w = (c & 2) ? w1 + 4 * (c & 1) : w0 + 4 * (c & 1);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sm + ws_swz(trow, thalf * 4 + c)), "r"(w[0]),
+                             "r"(w[1]), "r"(w[2]), "r"(w[3])
+                             : "memory");
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) ws_arrive(a_full + 8 * sA);
+            // The chunk is given back only here, after its words have gone through registers into the stores above: with the
+            // arrival right behind the loads the copy engine overwrote words that a load still had to read.
+            if (LAYOUT == kTiled && (a.mh == 1 || (i & 1))) {
+                if (lane == 0) ws_arrive(w_free + 8 * cw.s);
+                cw.advance(a.sw);
+            }
+        }
+        if (!ok && lane == 0) ws_count_timeout(a.timeouts);
+    }
+    __syncwarp();
+    // ---- epilogue: accumulators -> shared memory, [column][128 rows] words in place of the rings -> output.  Every
+    //      thread of the block then takes four rows of a column: the output is written 256 (512) bytes at a time.  In a
+    //      cluster block z adds and stores the columns [z cs, + cs) of all blocks' sums.
+    grid_dep_wait();  // the output may still be read by a predecessor, the scales are its result
+    if (HALF_OUT && tid < a.nt) scales[tid] = dequant_scale(m.gamma, a.absmax[min(n0 + tid, a.n - 1)]);
+    if (warp < kWsExpandWarps) {
+        ok = ws_wait(done_b, 0, a.wait_cycles) && ok;
+        ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
+        if (!ok && lane == 0) ws_count_timeout(a.timeouts);
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncthreads();  // every copy has landed and every MMA is done (or a wait ran out: the output is unspecified)
+    const bool vec_out = m.rows % 4 == 0 && (reinterpret_cast<uintptr_t>(m.out) & (HALF_OUT ? 7u : 15u)) == 0;
+    const int S = a.split, cs = (a.nt + S - 1) / S, me = static_cast<int>(blockIdx.z);
+    for (int g = 0; g < a.mh; ++g) {
+        if (warp < kWsExpandWarps && ok)  // tensor-memory lanes 32 (w % 4) .. + 31, 16 columns at a time
+            for (int c0 = 16 * (warp >> 2); c0 < a.nt; c0 += 64) {
+                uint32_t r[16];
+                const uint32_t taddr = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(g * a.nt + c0);
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                    : "r"(taddr)
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const uint32_t at = ring_s + static_cast<uint32_t>((c0 * kWsTileM + (warp & 3) * 32 + lane) * 4);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + i * kWsTileM * 4), "r"(r[i]) : "memory");
+            }
+        if (S > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+        const int c_lo = me * cs, c_hi = min(a.nt, c_lo + cs);
+        for (int e = c_lo * 32 + tid; e < c_hi * 32; e += static_cast<int>(blockDim.x)) {
+            const int c = e >> 5, row = row0 + g * kWsTileM + 4 * (e & 31), j = n0 + c;
+            const uint32_t at = ring_s + static_cast<uint32_t>(e) * 16;
+            int4 sum;
+            if (S == 1) {
+                asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(sum.x), "=r"(sum.y), "=r"(sum.z), "=r"(sum.w) : "r"(at) : "memory");
+            } else {
+                sum = make_int4(0, 0, 0, 0);
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+                    if (p < S) {
+                        uint32_t remote;
+                        int4 v;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(p));
+                        asm volatile("ld.shared::cluster.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote));
+                        sum.x += v.x;
+                        sum.y += v.y;
+                        sum.z += v.z;
+                        sum.w += v.w;
+                    }
+            }
+            if (j >= a.n || row >= m.rows) continue;
+            const size_t o = static_cast<size_t>(j) * m.rows + row;
+            if (HALF_OUT) {
+                const float sc = scales[c];
+                __half h[4];
+                h[0] = __float2half_rn(__fmul_rn(static_cast<float>(sum.x), sc));
+                h[1] = __float2half_rn(__fmul_rn(static_cast<float>(sum.y), sc));
+                h[2] = __float2half_rn(__fmul_rn(static_cast<float>(sum.z), sc));
+                h[3] = __float2half_rn(__fmul_rn(static_cast<float>(sum.w), sc));
+                __half* dst = static_cast<__half*>(m.out) + o;
+                if (vec_out) {
+                    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (row + i < m.rows) dst[i] = h[i];
+                }
+            } else {
+                int32_t* dst = static_cast<int32_t*>(m.out) + o;
+                if (vec_out) {
+                    *reinterpret_cast<int4*>(dst) = sum;
+                } else {
+                    const int32_t v[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (row + i < m.rows) dst[i] = v[i];
+                }
+            }
+        }
+        if (S > 1) {  // nobody leaves, or overwrites its sums, while a peer reads them
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else if (g + 1 < a.mh) {
+            __syncthreads();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -413,69 +648,158 @@ void prepare_host_state() {
     sm_count();
 }
 
-// Launch of the warp-specialised form; the caller has checked the layout (cols % 128 == 0, aligned rows and X).
-// Returns SPB_E_UNSUPPORTED when the tensor map of X cannot be made (the caller then takes the plain form).
-int gemm_tcsp_ws_launch(const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y, int rows, int cols,
-                        int n, int meta_stride, int values_stride, void* stream, const GemmEpilogue* ep) {
-    WsArgs a{};
-    a.meta = meta; a.values = values; a.Y = Y;
-    if (ep) a.ep = *ep;
-    a.rows = rows; a.cols = cols; a.n = n;
-    a.meta_stride = meta_stride; a.values_stride = values_stride;
-    // batch rows per block: 256, or 128 / 64 when the wider tile would leave more than half of the SMs without a
-    // block (a step costs about the same whatever the tile width, so more, narrower blocks finish sooner)
-    const int mtiles = (rows + kWsTileM - 1) / kWsTileM;
-    int nt = 256;
-    while (nt > 64 && mtiles * ((n + nt - 1) / nt) < sm_count() / 2) nt >>= 1;
-    a.nt = min(nt, (n + 15) / 16 * 16);
-    // Two row halves per block (256 weight rows on one activation tile, one re-encoding group per half, two
-    // accumulators).  A step then costs about twice as much (the MMA warp issues eight MMAs, each group re-encodes
-    // every step), so it only pays by saving a wave.  Both accumulators and the metadata slots must fit the 512
-    // tensor-memory columns: 240 batch rows.
-    a.mh = 1;
-    if (g_ws_mh != 1 && n > 128) {
-        // automatic: only where the 128-row blocks need a second wave and the 256-row blocks fit into one
-        // (measured: 6912x2560 at n = 1024, 25.2 -> 22.1 us; everywhere else the 128-row form is faster)
-        const int mt2 = (rows + 2 * kWsTileM - 1) / (2 * kWsTileM), nt2 = 240;
-        const int items1 = mtiles * ((n + a.nt - 1) / a.nt), items2 = mt2 * ((n + nt2 - 1) / nt2);
-        if (g_ws_mh == 2 || (items1 > sm_count() && items2 <= sm_count() && items2 >= (3 * sm_count()) / 4)) {
-            a.mh = 2;
-            a.nt = min(nt2, (n + 15) / 16 * 16);
+static bool ws_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int inner, int outer,
+                   size_t stride_bytes, int box_inner, int box_outer, CUtensorMapSwizzle swizzle) {
+    const EncodeFn encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
+    const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(stride_bytes)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
+    const cuuint32_t estr[2] = {1u, 1u};
+    return encode(map, type, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+struct WsShape {
+    int mh, nt, split, sa, sb, sw;
+    size_t smem;
+};
+
+// Ring depths for a tile: as many stages as fit, the activations first (their latency is the longest after the weights').
+static void ws_rings(WsShape& c, bool tiled) {
+    const int ab = c.mh * kWsABytes, bb = c.nt * 128, wb = tiled ? c.mh * kWsWBytes : 0;
+    c.sa = 2;
+    c.sb = 2;
+    c.sw = tiled ? 2 : 0;
+    const int cap = kWsSmemCap - kWsBarBytes - kWsScaleBytes - 1024;
+    auto used = [&] { return c.sa * ab + c.sb * bb + c.sw * wb; };
+    for (bool grew = true; grew;) {
+        grew = false;
+        if (c.sb < 4 && used() + bb <= cap) { ++c.sb; grew = true; }
+        if (tiled && c.sw < 4 && used() + wb <= cap) { ++c.sw; grew = true; }
+        if (c.sa < 4 && c.mh * (c.nt + 8 * (c.sa + 1)) <= 512 && used() + ab <= cap) { ++c.sa; grew = true; }
+    }
+    // the epilogue's sums take the place of the rings
+    c.smem = kWsBarBytes + kWsScaleBytes + 1024 + static_cast<size_t>(max(used(), c.nt * kWsTileM * 4));
+}
+
+// How a product is cut: 128- or 256-row blocks, batch rows per block, blocks per cluster along K: the least of
+//   waves * (start + steps * clocks per step + drain [+ exchange])
+// in clocks, as measured (nt = batch rows per block, clocks per step of 256 columns):
+//   128 rows: 690 up to nt = 128 (re-encoding), 925 at 176, 1047 at 256 (activations out of L2, 62 B per clock and SM);
+//   256 rows: 1250 at nt = 64 (re-encoding), 1530 at 208: half the activation traffic per weight row, so it wins where
+//   the batch is wide, and where it saves a wave;
+//   start: 4500 to the first product (weights from HBM, re-encoding, activations);
+//   drain: 9 per batch row to stage the sums, 16 to write them out;
+//   exchange: two cluster barriers and (S - 1) / S of the sums at 13 B per clock, in place of writing them all out.
+static WsShape ws_choose(const TcspMat* mats, int nmat, int cols, int n, bool tiled) {
+    const int sms = sm_count();
+    const int steps = (cols + kWsStepK - 1) / kWsStepK;
+    WsShape best{};
+    double best_cost = 1e30;
+    for (int mh = 1; mh <= (tiled ? 2 : 1); ++mh) {
+        if (g_ws_mh && tiled && mh != g_ws_mh) continue;
+        long long tiles = 0;
+        for (int i = 0; i < nmat; ++i) tiles += (mats[i].rows + mh * kWsTileM - 1) / (mh * kWsTileM);
+        const int max_nt = mh == 2 ? 240 : 256;
+        const int first = (n + max_nt - 1) / max_nt;
+        for (int nn = first; nn <= first + 3; ++nn) {
+            const int nt = ((n + nn - 1) / nn + 15) / 16 * 16;
+            if (nt > max_nt || (nn > first && nt < 64)) continue;
+            const long long blocks = tiles * ((n + nt - 1) / nt);
+            const double step = mh == 2 ? fmax(1250.0, 370.0 + 5.6 * nt) : fmax(690.0, 330.0 + 2.8 * nt);
+            for (int S = 1; S <= (mh == 1 ? 8 : 1) && S <= steps; ++S) {
+                // a cluster sits in one GPC: groups of five to eight leave some of its 18 or so SMs idle
+                const int slots = S <= 2 ? sms : S <= 4 ? sms * 15 / 16 : sms * 7 / 8;
+                const double waves = ceil(static_cast<double>(blocks) * S / slots);
+                const double out = S > 1 ? 2800.0 + 36.0 * nt * (S - 1) / S : 16.0 * nt * mh;
+                const double cost = waves * (4500.0 + (steps + S - 1) / S * step + 9.0 * nt * mh + out);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best.mh = mh;
+                    best.nt = nt;
+                    best.split = S;
+                }
+            }
         }
     }
-    const int stage_bytes = a.mh * kWsABytes + 2 * a.nt * 128;
-    a.stages = max(2, min(kWsMaxStages, (200 * 1024) / stage_bytes));
-    // two groups pay off except at 128 batch rows per block (measured at 6912x2560, n = 256: 12.4 against 11.9 us)
-    a.groups = a.mh == 2 ? 2 : a.nt == 128 ? 1 : 2;
-    // A group must not run more than one ring revolution ahead of the MMA warp, or its parity wait on a stage's
-    // "free" barrier would be satisfied by the previous completion of the same parity.  A group's wait for step k
-    // confirms the commit of step k - stages; its next step is k + groups, whose wait needs the commit of
-    // k + groups - 2 * stages to be over: true when groups <= stages.  (Three groups on two stages were tried and
-    // ran into exactly this.)
-    a.groups = min(a.groups, a.stages);
+    ws_rings(best, tiled);
+    return best;
+}
+
+int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const float* absmax, int cols, int n, void* stream) {
+    const char* name = "spb_sparse_ternary_gemm(tcgen05.sp)";
+    auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    bool tiled = cols % 16 == 0 && al(X);
+    for (int i = 0; i < nmat; ++i)
+        tiled = tiled && al(mats[i].meta) && al(mats[i].values) && mats[i].meta_stride % 4 == 0 && mats[i].values_stride % 4 == 0;
+    WsArgs a{};
+    alignas(64) WsMaps maps;
+    WsShape c = ws_choose(mats, nmat, cols, n, tiled);
+    auto encode_all = [&] {
+        bool good = ws_map(&maps.x, CU_TENSOR_MAP_DATA_TYPE_UINT8, X, cols, n, cols, 128, c.nt, CU_TENSOR_MAP_SWIZZLE_128B);
+        for (int i = 0; i < nmat && good; ++i)
+            good = ws_map(&maps.meta[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, mats[i].meta, (cols + 31) / 32, mats[i].rows,
+                          static_cast<size_t>(mats[i].meta_stride) * 4, 16, c.mh * kWsTileM, CU_TENSOR_MAP_SWIZZLE_64B) &&
+                   ws_map(&maps.values[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, mats[i].values, (cols + 63) / 64, mats[i].rows,
+                          static_cast<size_t>(mats[i].values_stride) * 4, 8, c.mh * kWsTileM, CU_TENSOR_MAP_SWIZZLE_32B);
+        return good;
+    };
+    if (tiled && !encode_all()) {
+        tiled = false;
+        c = ws_choose(mats, nmat, cols, n, tiled);
+    }
+    if (!tiled) memset(&maps, 0, sizeof maps);
+    a.X = X;
+    a.absmax = absmax;
+    a.nmat = nmat;
+    a.cols = cols;
+    a.n = n;
+    a.nt = c.nt;
+    a.mh = c.mh;
+    a.sa = c.sa;
+    a.sb = c.sb;
+    a.sw = c.sw;
+    a.split = c.split;
+    int tiles = 0;
+    for (int i = 0; i < nmat; ++i) {
+        a.m[i] = WsMat{mats[i].meta, mats[i].values, mats[i].out, mats[i].gamma, mats[i].rows, mats[i].meta_stride,
+                       mats[i].values_stride, tiles};
+        tiles += (mats[i].rows + c.mh * kWsTileM - 1) / (c.mh * kWsTileM);
+    }
     a.tmem_cols = 32;
-    while (a.tmem_cols < a.mh * (a.nt + 8 * a.stages)) a.tmem_cols <<= 1;
-    if (a.tmem_cols > 512) return fail(SPB_E_UNSUPPORTED, "gemm_tcsp_ws: %d tensor-memory columns", a.tmem_cols);
-    const size_t smem = kWsSignLutBytes + 128 + 1024 + static_cast<size_t>(a.stages) * stage_bytes;
-    const EncodeFn encode = tensor_map_encoder();
-    if (!encode) return SPB_E_UNSUPPORTED;
-    // tensor map of X: uint8 [n rows][cols], box 128 bytes x nt rows, 128-byte swizzle, zero fill past n
-    alignas(64) CUtensorMap tmap;
-    const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(n)};
-    const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(cols)};
-    const cuuint32_t box[2] = {128u, static_cast<cuuint32_t>(a.nt)};
-    const cuuint32_t estr[2] = {1u, 1u};
-    if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(X), gdim, gstride, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return SPB_E_UNSUPPORTED;
-    void (*kernel)(WsArgs, CUtensorMap) = a.ep.out ? gemm_tcsp_ws_kernel<true> : gemm_tcsp_ws_kernel<false>;
-    if (int rc = ensure_dynamic_smem("gemm_tcsp_ws", kernel, smem)) return rc;
+    while (a.tmem_cols < c.mh * (c.nt + 8 * c.sa)) a.tmem_cols <<= 1;
     a.timeouts = timeout_counter();
     a.wait_cycles = kWsWaitCycles;
-    const dim3 grid((rows + a.mh * kWsTileM - 1) / (a.mh * kWsTileM), (n + a.nt - 1) / a.nt);
-    return launch("spb_sparse_ternary_gemm(tcgen05.sp, warp-specialised)", kernel, grid, dim3(kWsThreads), smem,
-                  stream, a, tmap);
+    using Kernel = void (*)(WsArgs, WsMaps);
+    const Kernel kernel = tiled ? (absmax ? gemm_tcsp_ws_kernel<true, kTiled> : gemm_tcsp_ws_kernel<false, kTiled>)
+                                : (absmax ? gemm_tcsp_ws_kernel<true, kAny> : gemm_tcsp_ws_kernel<false, kAny>);
+    if (int rc = ensure_dynamic_smem(name, kernel, c.smem)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles, (n + c.nt - 1) / c.nt, c.split);
+    cfg.blockDim = dim3(tiled ? kWsThreadsTiled : kWsThreadsAny);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (pdl_enabled()) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (c.split > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = 1;
+        attr[na].val.clusterDim.y = 1;
+        attr[na++].val.clusterDim.z = c.split;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, a, maps);
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SPB_E_CUDA, "%s: launch failed: %s", name, cudaGetErrorString(err));
+    }
+    return SPB_OK;
 }
 
 }  // namespace spb

@@ -1,0 +1,53 @@
+"""The tcgen05 product at the edges of its tiles and of its split: row and batch tails, one step of K and ranges that do not
+divide over a cluster, widths that are no multiple of a word, unaligned operands.  Integer sums: exact."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from spbitnet_b200 import kernels as K, synth
+from gpu_util import Guarded, dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def tcgen05_form():
+    old = K.set_gemm_variant(3)
+    before = K.gemm_tc_timeouts()
+    yield
+    K.set_gemm_variant(old)
+    assert K.gemm_tc_timeouts() == before
+
+
+@pytest.mark.parametrize("rows,cols,n", [(1, 4, 1), (128, 256, 16), (127, 512, 17), (129, 768, 1), (130, 2560, 15),
+                                         (256, 16384, 3), (640, 2304, 65), (384, 6912, 200), (20, 28672, 24),
+                                         (300, 272, 33), (301, 132, 40), (37, 3204, 129), (513, 1036, 257)])
+def test_sums_and_scaled_half(rows, cols, n):
+    case = synth.gemm_case(rows, cols, n, seed=rows * 31 + n)
+    want = oracle.sparse_gemm(case["meta"], case["values"], case["X"], rows, cols)
+    Y = Guarded(n * rows * 4)
+    K.sparse_ternary_gemm_gpu(dev(case["meta"]), dev(case["values"]), dev(case["X"]), Y.ptr, rows, cols, n,
+                              case["meta_stride"], case["values_stride"])
+    assert (Y.read(np.int32).reshape(n, rows) == want).all()
+    out, ws = Guarded(n * rows * 2), Guarded(n * rows * 4)
+    K.sparse_bitlinear_gemm_gpu(dev(case["meta"]), dev(case["values"]), dev(case["X"]), out.ptr, dev(case["absmax"]), 0.05,
+                                rows, cols, n, case["meta_stride"], case["values_stride"], acc_workspace=ws.ptr)
+    wh = np.stack([oracle.dequantize(want[j], case["absmax"][j], np.float32(0.05)) for j in range(n)])
+    assert (out.read(np.float16).reshape(n, rows).view(np.uint16) == wh.view(np.uint16)).all()
+
+
+def test_unaligned_operands_and_padded_rows():
+    rows, cols, n = 150, 640, 21
+    case = synth.gemm_case(rows, cols, n, seed=4)
+    want = oracle.sparse_gemm(case["meta"], case["values"], case["X"], rows, cols)
+    ms, vs = case["meta_stride"], case["values_stride"]
+    for pad_m, pad_v, shift in [(4, 2, 0), (1, 3, 0), (0, 0, 1), (12, 10, 3)]:
+        meta = np.full((rows, ms + pad_m), 0xFFFFFFFF, np.uint32)  # the padding is never used
+        values = np.full((rows, vs + pad_v), 0xFFFFFFFF, np.uint32)
+        meta[:, :ms], values[:, :vs] = case["meta"], case["values"]
+        x = torch.zeros(n * cols + 16, dtype=torch.int8, device="cuda")
+        x[shift:shift + n * cols] = dev(case["X"]).flatten()
+        Y = Guarded(n * rows * 4, align_offset=4 * shift)
+        K.sparse_ternary_gemm_gpu(dev(meta), dev(values), x.data_ptr() + shift, Y.ptr, rows, cols, n, ms + pad_m, vs + pad_v)
+        assert (Y.read(np.int32).reshape(n, rows) == want).all(), (pad_m, pad_v, shift)
