@@ -165,6 +165,18 @@ def load() -> C.CDLL:
     return lib
 
 
+def calls():
+    """The CPython module that calls the kernel entry points (csrc/py_calls.cpp), bound to the loaded library."""
+    lib = load()
+    try:
+        from . import _calls
+    except ImportError as e:
+        raise ImportError("spbitnet_b200/_calls is missing. Build it with `python -m spbitnet_b200.build`.") from e
+    _calls.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES},
+                check)
+    return _calls
+
+
 def check(status: int) -> None:
     if status != SPB_OK:
         raise SpbError(status, load().spb_last_error_string().decode("utf-8", "replace"))

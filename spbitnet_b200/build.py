@@ -8,6 +8,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -15,7 +16,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "libspbitnet_b200.so"
 CLI = HERE / "spbitnet_infer"
-SOURCES = ["core.cu", "gemv.cu", "gemv_batch_mma.cu", "gemv_mmasp.cu", "gemv_prepared.cu", "gemm.cu", "gemm_tcsp_ws.cu", "gemm_mmasp.cu", "unpack.cu",
+CALLS = HERE / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+SOURCES = ["core.cu", "gemv.cu", "gemv_batch_mma.cu", "gemv_mmasp.cu", "gemv_prepared.cu", "gemm.cu", "gemm_tcsp_ws.cu", "half_gemm_tc.cu", "gemm_mmasp.cu", "unpack.cu",
            "decode_ops.cu", "attention.cu", "attention_prefill.cu", "fused_ops.cu", "prefill.cu", "decode_persistent.cu", "engine.cu", "sharded.cu", "noalloc.cu", "pack.cu", "format_host.cpp",
            "tokenizer.cpp", "model_loader.cpp"]
 COMPILE_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -36,7 +38,7 @@ def sources() -> list[Path]:
 
 
 def needs_build() -> bool:
-    if not LIB.exists():
+    if not LIB.exists() or not CALLS.exists():
         return True
     t = LIB.stat().st_mtime
     deps = [p for p in CSRC.glob("*") if p.is_file()] + [HERE.parent / "include" / "spbitnet_b200.h"]
@@ -75,6 +77,13 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     res = subprocess.run([nvcc, *LINK_FLAGS, "-o", str(LIB), *objs], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    # the CPython module that calls the entry points (bound to the loaded library at import, not linked)
+    calls_src = CSRC / "py_calls.cpp"
+    if force or not CALLS.exists() or CALLS.stat().st_mtime < max(calls_src.stat().st_mtime, newest_header):
+        res = subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-I",
+                              sysconfig.get_paths()["include"], "-o", str(CALLS), str(calls_src)], capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"building {CALLS.name} failed:\n{res.stdout}\n{res.stderr}")
     # the command line (the reference's spbitnet_infer, src/main.cpp) on top of the library
     cli_src = CSRC / "cli_main.cpp"
     if force or not CLI.exists() or CLI.stat().st_mtime < max(cli_src.stat().st_mtime, LIB.stat().st_mtime):

@@ -1,7 +1,7 @@
 """Python mirror of the reference's kernel host wrappers (namespace spbitnet,
 include/spbitnet/sparse_ternary_kernels.h and inference_kernels.h): same names, same
 argument order, torch CUDA tensors in place of device pointers.  Every function forwards
-to the C-ABI of libspbitnet_b200.so; errors raise SpbError instead of exiting.
+to the C-ABI of libspbitnet_b200.so (through the CPython module `_calls`); errors raise SpbError instead of exiting.
 """
 from __future__ import annotations
 
@@ -9,7 +9,10 @@ import ctypes as C
 
 import torch
 
+from . import _lib
 from ._lib import check, load
+
+_c = _lib.calls()  # converts tensors, addresses, None and streams; a status other than 0 raises SpbError
 
 
 def _p(t):
@@ -66,13 +69,11 @@ def debug_grid_barrier_selftest(limit_cycles: int = 200000, stream=None) -> int:
 # ---- sparse_ternary_kernels.h ---------------------------------------------------------
 
 def sparse_ternary_unpack_gpu(meta, values, out, rows, cols, meta_row_stride, values_row_stride, stream=None):
-    check(load().spb_sparse_ternary_unpack(_p(meta), _p(values), _p(out), rows, cols, meta_row_stride,
-                                           values_row_stride, _stream(stream)))
+    _c.spb_sparse_ternary_unpack(meta, values, out, rows, cols, meta_row_stride, values_row_stride, stream)
 
 
 def sparse_ternary_gemv_gpu(meta, values, x, y, rows, cols, meta_row_stride, values_row_stride, stream=None):
-    check(load().spb_sparse_ternary_gemv(_p(meta), _p(values), _p(x), _p(y), rows, cols, meta_row_stride,
-                                         values_row_stride, _stream(stream)))
+    _c.spb_sparse_ternary_gemv(meta, values, x, y, rows, cols, meta_row_stride, values_row_stride, stream)
 
 
 def prepared_weights_bytes(rows, cols) -> int:
@@ -85,18 +86,16 @@ def prepare_weights(meta, values, rows, cols, meta_row_stride, values_row_stride
     if nbytes == 0:
         raise ValueError(f"prepared weights: shape {rows}x{cols} not taken (cols must be a multiple of 256)")
     out = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
-    check(load().spb_prepare_weights(_p(meta), _p(values), rows, cols, meta_row_stride, values_row_stride, _p(out),
-                                     _stream(stream)))
+    _c.spb_prepare_weights(meta, values, rows, cols, meta_row_stride, values_row_stride, out, stream)
     return out
 
 
 def prepared_gemv_gpu(prepared, x, y, rows, cols, stream=None):
-    check(load().spb_prepared_gemv(_p(prepared), _p(x), _p(y), rows, cols, _stream(stream)))
+    _c.spb_prepared_gemv(prepared, x, y, rows, cols, stream)
 
 
 def prepared_bitlinear_q8_gpu(prepared, xq, out_half, d_absmax, gamma, rows, cols, stream=None):
-    check(load().spb_prepared_bitlinear_q8(_p(prepared), _p(xq), _p(out_half), _p(d_absmax), float(gamma), rows, cols,
-                                           _stream(stream)))
+    _c.spb_prepared_bitlinear_q8(prepared, xq, out_half, d_absmax, gamma, rows, cols, stream)
 
 
 class GemvWorkList:
@@ -121,32 +120,29 @@ class GemvWorkList:
 
 
 def sparse_ternary_gemv_batch_gpu(work: GemvWorkList, stream=None):
-    check(load().spb_sparse_ternary_gemv_batch(_p(work.d_items), work.n, work.max_rows, work.max_cols,
-                                               _stream(stream)))
+    _c.spb_sparse_ternary_gemv_batch(work.d_items, work.n, work.max_rows, work.max_cols, stream)
 
 
 def sparse_ternary_gemv_scaled_gpu(meta, values, x, y, y_acc, d_absmax, gamma, rows, cols, meta_row_stride,
                                    values_row_stride, stream=None):
-    check(load().spb_sparse_ternary_gemv_scaled(_p(meta), _p(values), _p(x), _p(y), _p(y_acc), _p(d_absmax),
-                                                float(gamma), rows, cols, meta_row_stride, values_row_stride,
-                                                _stream(stream)))
+    _c.spb_sparse_ternary_gemv_scaled(meta, values, x, y, y_acc, d_absmax, gamma, rows, cols, meta_row_stride,
+                                      values_row_stride, stream)
 
 
 def fused_sparse_bitlinear_gpu(meta, values, x, output, d_absmax, gamma, rows, cols, meta_row_stride,
                                values_row_stride, stream=None):
-    check(load().spb_fused_sparse_bitlinear(_p(meta), _p(values), _p(x), _p(output), _p(d_absmax), float(gamma),
-                                            rows, cols, meta_row_stride, values_row_stride, _stream(stream)))
+    _c.spb_fused_sparse_bitlinear(meta, values, x, output, d_absmax, gamma, rows, cols, meta_row_stride,
+                                  values_row_stride, stream)
 
 
 def sparse_bitlinear_q8_gpu(meta, values, xq, output, d_absmax, gamma, rows, cols, meta_row_stride,
                             values_row_stride, stream=None):
-    check(load().spb_sparse_bitlinear_q8(_p(meta), _p(values), _p(xq), _p(output), _p(d_absmax), float(gamma),
-                                         rows, cols, meta_row_stride, values_row_stride, _stream(stream)))
+    _c.spb_sparse_bitlinear_q8(meta, values, xq, output, d_absmax, gamma, rows, cols, meta_row_stride,
+                               values_row_stride, stream)
 
 
 def sparse_ternary_gemm_gpu(meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream=None):
-    check(load().spb_sparse_ternary_gemm(_p(meta), _p(values), _p(X), _p(Y), rows, cols, n, meta_row_stride,
-                                         values_row_stride, _stream(stream)))
+    _c.spb_sparse_ternary_gemm(meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream)
 
 
 def sparse_bitlinear_gemm_gpu(meta, values, Xq, output, d_absmax, gamma, rows, cols, n, meta_row_stride,
@@ -154,57 +150,54 @@ def sparse_bitlinear_gemm_gpu(meta, values, Xq, output, d_absmax, gamma, rows, c
     """BitLinear over n quantised activation rows (no counterpart in the reference, whose prefill is token-serial):
     output[j] = half(float(W @ Xq[j]) * (gamma * d_absmax[j] / 127)).  acc_workspace: n * rows int32, needed only by
     the forms without a fused epilogue."""
-    ws = _p(acc_workspace) if acc_workspace is not None else None
-    check(load().spb_sparse_bitlinear_gemm(_p(meta), _p(values), _p(Xq), _p(output), _p(d_absmax), float(gamma), ws,
-                                           rows, cols, n, meta_row_stride, values_row_stride, _stream(stream)))
+    _c.spb_sparse_bitlinear_gemm(meta, values, Xq, output, d_absmax, gamma, acc_workspace, rows, cols, n, meta_row_stride,
+                                 values_row_stride, stream)
 
 
 # ---- inference_kernels.h ----------------------------------------------------------------
 
 def rms_norm_gpu(input, weight, output, size, eps, stream=None):
-    check(load().spb_rms_norm(_p(input), _p(weight), _p(output), size, float(eps), _stream(stream)))
+    _c.spb_rms_norm(input, weight, output, size, eps, stream)
 
 
 def absmax_quantize_gpu(input, output, d_absmax, size, stream=None):
-    check(load().spb_absmax_quantize(_p(input), _p(output), _p(d_absmax), size, _stream(stream)))
+    _c.spb_absmax_quantize(input, output, d_absmax, size, stream)
 
 
 def absmax_reduce_gpu(input, d_absmax, size, stream=None):
-    check(load().spb_absmax_reduce(_p(input), _p(d_absmax), size, _stream(stream)))
+    _c.spb_absmax_reduce(input, d_absmax, size, stream)
 
 
 def dequantize_gpu(input, output, d_absmax, gamma, size, stream=None):
-    check(load().spb_dequantize(_p(input), _p(output), _p(d_absmax), float(gamma), size, _stream(stream)))
+    _c.spb_dequantize(input, output, d_absmax, gamma, size, stream)
 
 
 def rope_gpu(vec, num_heads, head_dim, pos, theta, stream=None):
-    check(load().spb_rope(_p(vec), num_heads, head_dim, pos, float(theta), _stream(stream)))
+    _c.spb_rope(vec, num_heads, head_dim, pos, theta, stream)
 
 
 def scatter_kv_gpu(src, cache, num_kv_heads, head_dim, max_seq_len, pos, stream=None):
-    check(load().spb_scatter_kv(_p(src), _p(cache), num_kv_heads, head_dim, max_seq_len, pos, _stream(stream)))
+    _c.spb_scatter_kv(src, cache, num_kv_heads, head_dim, max_seq_len, pos, stream)
 
 
 def attention_scores_gpu(Q, K_cache, scores, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len, scale,
                          stream=None):
-    check(load().spb_attention_scores(_p(Q), _p(K_cache), _p(scores), num_heads, num_kv_heads, head_dim,
-                                      max_seq_len, seq_len, float(scale), _stream(stream)))
+    _c.spb_attention_scores(Q, K_cache, scores, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len, scale, stream)
 
 
 def softmax_gpu(scores, num_heads, max_seq_len, seq_len, stream=None):
-    check(load().spb_softmax(_p(scores), num_heads, max_seq_len, seq_len, _stream(stream)))
+    _c.spb_softmax(scores, num_heads, max_seq_len, seq_len, stream)
 
 
 def attention_output_gpu(scores, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len,
                          stream=None):
-    check(load().spb_attention_output(_p(scores), _p(V_cache), _p(output), num_heads, num_kv_heads, head_dim,
-                                      max_seq_len, seq_len, _stream(stream)))
+    _c.spb_attention_output(scores, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len, stream)
 
 
 def decode_attention_gpu(Q, K_cache, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len,
                          scale, stream=None):
-    check(load().spb_decode_attention(_p(Q), _p(K_cache), _p(V_cache), _p(output), num_heads, num_kv_heads,
-                                      head_dim, max_seq_len, seq_len, float(scale), _stream(stream)))
+    _c.spb_decode_attention(Q, K_cache, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len, scale,
+                            stream)
 
 
 def decode_attention_scratch_bytes(num_heads, head_dim, max_seq_len) -> int:
@@ -214,33 +207,32 @@ def decode_attention_scratch_bytes(num_heads, head_dim, max_seq_len) -> int:
 def decode_attention_split_gpu(Q, K_cache, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len,
                                scale, scratch, stream=None):
     nbytes = scratch.numel() * scratch.element_size()
-    check(load().spb_decode_attention_split(_p(Q), _p(K_cache), _p(V_cache), _p(output), num_heads, num_kv_heads,
-                                            head_dim, max_seq_len, seq_len, float(scale), _p(scratch), nbytes,
-                                            _stream(stream)))
+    _c.spb_decode_attention_split(Q, K_cache, V_cache, output, num_heads, num_kv_heads, head_dim, max_seq_len, seq_len,
+                                  scale, scratch, nbytes, stream)
 
 
 def relu2_mul_gpu(gate, up, output, size, stream=None):
-    check(load().spb_relu2_mul(_p(gate), _p(up), _p(output), size, _stream(stream)))
+    _c.spb_relu2_mul(gate, up, output, size, stream)
 
 
 def relu2_mul_f32_gpu(gate, up, output, size, stream=None):
-    check(load().spb_relu2_mul_f32(_p(gate), _p(up), _p(output), size, _stream(stream)))
+    _c.spb_relu2_mul_f32(gate, up, output, size, stream)
 
 
 def rms_norm_f32in_gpu(input, weight, output, size, eps, stream=None):
-    check(load().spb_rms_norm_f32in(_p(input), _p(weight), _p(output), size, float(eps), _stream(stream)))
+    _c.spb_rms_norm_f32in(input, weight, output, size, eps, stream)
 
 
 def float_to_half_gpu(input, output, size, stream=None):
-    check(load().spb_float_to_half(_p(input), _p(output), size, _stream(stream)))
+    _c.spb_float_to_half(input, output, size, stream)
 
 
 def residual_add_gpu(a, b, output, size, stream=None):
-    check(load().spb_residual_add(_p(a), _p(b), _p(output), size, _stream(stream)))
+    _c.spb_residual_add(a, b, output, size, stream)
 
 
 def half_gemv_gpu(W, x, y, rows, cols, stream=None):
-    check(load().spb_half_gemv(_p(W), _p(x), _p(y), rows, cols, _stream(stream)))
+    _c.spb_half_gemv(W, x, y, rows, cols, stream)
 
 
 # ---- conversion on the GPU (no counterpart among the reference's GPU wrappers) -----------------
@@ -257,7 +249,6 @@ def prune_pack_gpu(weights, stream=None):
     meta = torch.zeros((rows, ms), dtype=torch.int32, device=weights.device)
     values = torch.zeros((rows, vs), dtype=torch.int32, device=weights.device)
     abs_sum = torch.zeros(1, dtype=torch.float64, device=weights.device)
-    check(load().spb_prune_pack_gpu(_p(weights), rows, cols, weights.stride(0), _p(meta), _p(values), ms, vs,
-                                    _p(abs_sum), _stream(stream)))
+    _c.spb_prune_pack_gpu(weights, rows, cols, weights.stride(0), meta, values, ms, vs, abs_sum, stream)
     gamma = float(abs_sum.item()) / max(1, rows * cols)
     return meta, values, gamma
