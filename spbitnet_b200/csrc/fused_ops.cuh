@@ -64,6 +64,8 @@ int set_int(int* dst, int value, void* stream);
 // prefill.cu: row-batched forms, one block per token of the batch
 int embed_rows(const void* embed, const int* d_tokens, void* x, int hidden, int vectors, void* stream);
 int absmax_quantize_rows(const void* in, int8_t* out, float* d_absmax, int n, int vectors, void* stream);
+// half_gemm_tc.cu: y[b, r] = W[r] . x[b] for up to 64 half vectors, fp32 sums
+int half_gemm_tc(const __half* W, const __half* x, float* y, int rows, int cols, int batch, void* stream);
 int dequantize_rows(const int32_t* acc, void* out, const float* d_absmax, float gamma, int rows, int vectors,
                     void* stream);
 

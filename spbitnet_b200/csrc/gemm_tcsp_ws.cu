@@ -30,12 +30,11 @@
 //
 // Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run out of their own
 // bounds, the copy warps wait (bounded) for their copies in flight, tensor memory is freed and the block returns.
-#include <cuda.h>
-
 #include <cmath>
 #include <cstring>
 
 #include "gemm_tcsp_ws.cuh"
+#include "tcgen05_ops.cuh"
 
 namespace spb {
 
@@ -50,7 +49,6 @@ constexpr int kWsCopyWarps = 8;                // kAny: warps 17 .. 24 copy the 
 constexpr int kWsThreadsAny = 32 * (kWsXWarp + kWsCopyWarps);
 constexpr int kWsMaxRing = 8;
 constexpr int kWsBarBytes = 512, kWsScaleBytes = 1024;
-constexpr long long kWsWaitCycles = 40000000;
 constexpr int kWsSmemCap = 226 * 1024;
 
 enum WsLayout { kTiled = 0, kAny = 1 };
@@ -82,89 +80,10 @@ struct WsMaps {
 // 0 automatic, 1 / 2 force one / two weight-row halves per block (spb_set_gemm_row_halves; testing and measurement)
 static int g_ws_mh = 0;
 
-__device__ __forceinline__ void ws_count_timeout(int* counter) {
-    if (counter) atomicAdd_system(counter, 1);
-}
-
-__device__ __forceinline__ uint32_t ws_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-// K-major, 128-byte swizzle: 8-row groups of 1024 B (SBO), 16-byte leading offset.
-__device__ __forceinline__ uint64_t ws_smem_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
-}
 // kind::i8 instruction descriptor with the sparse flag: S32 accumulate, signed 8-bit A and B, K-major.
 __device__ __forceinline__ uint32_t ws_idesc(int m, int n) {
     return (1u << 2) | (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
            (static_cast<uint32_t>(m >> 4) << 24);
-}
-// Bounded by time, not by polls (a poll may suspend for a while): kWsWaitCycles is about 20 ms at 2 GHz.
-__device__ __forceinline__ bool ws_wait(uint32_t mbar, uint32_t parity, long long limit) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(mbar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (clock64() - t0 > limit) return false;
-    }
-}
-__device__ __forceinline__ void ws_arrive(uint32_t mbar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ void ws_init(uint32_t mbar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
-}
-__device__ __forceinline__ void ws_expect(uint32_t mbar, int bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void ws_tma(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
-        : "memory");
-}
-__device__ __forceinline__ void ws_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-// Position in a ring of barriers: stage and phase, advanced without a division.
-struct WsCursor {
-    int s = 0;
-    uint32_t ph = 0;
-    __device__ __forceinline__ void advance(int depth, int by = 1) {
-        s += by;
-        if (s >= depth) {
-            s -= depth;
-            ph ^= 1u;
-        }
-    }
-};
-__device__ __forceinline__ bool ws_elect() {
-    uint32_t e;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xFFFFFFFF;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(e));
-    return e != 0;
 }
 // One MMA: 128 rows x N, 64 logical columns.  a_lo, b_lo: low words of the operands' descriptors.
 __device__ __forceinline__ void ws_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t meta) {
@@ -178,10 +97,6 @@ __device__ __forceinline__ void ws_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo,
         :
         : "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(meta), "r"(hi)
         : "memory");
-}
-// 16-byte piece c of row r of a 128-byte-swizzled tile
-__device__ __forceinline__ uint32_t ws_swz(int r, int c) {
-    return static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }
 // Bitmaps of zero (past the end of a row or of the matrix: the activations there are zero, the rows are not stored)
 // become {0, 1}: the tensor core is only given valid pairs.
@@ -648,7 +563,7 @@ void prepare_host_state() {
     sm_count();
 }
 
-static bool ws_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int inner, int outer,
+bool ws_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int inner, int outer,
                    size_t stride_bytes, int box_inner, int box_outer, CUtensorMapSwizzle swizzle) {
     const EncodeFn encode = tensor_map_encoder();
     if (!encode) return false;
