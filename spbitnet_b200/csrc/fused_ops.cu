@@ -9,6 +9,7 @@
 // The position is read from device memory so that one captured CUDA graph serves every
 // token of a sequence.
 #include "fused_ops.cuh"
+#include "row_ops.cuh"
 
 namespace spb {
 
@@ -366,6 +367,9 @@ static int fused_threads(int n) {
 
 int residual_norm_quant(const void* delta, const float* sub_w, void* x, const float* w, void* xn_out,
                         int8_t* xq, float* d_absmax, int n, float eps, void* stream, int vectors) {
+    if (row_ops_take(n, delta, sub_w, x, w, xn_out, xq))
+        return rows_residual_norm_quant(static_cast<const __half*>(delta), sub_w, static_cast<__half*>(x), w,
+                                        static_cast<__half*>(xn_out), xq, d_absmax, n, eps, stream, vectors);
     const size_t smem = sizeof(float) * static_cast<size_t>(n);
     if (smem > 200 * 1024) return fail(SPB_E_UNSUPPORTED, "residual_norm_quant: n=%d too large", n);
     if (smem > 48 * 1024) cudaFuncSetAttribute(residual_norm_quant_kernel,
@@ -377,6 +381,9 @@ int residual_norm_quant(const void* delta, const float* sub_w, void* x, const fl
 
 int relu2_norm_quant(const void* gate, const void* up, const float* sub_w, void* h_out, int8_t* hq,
                      float* d_absmax, int n, float eps, void* stream, int vectors) {
+    if (row_ops_take(n, gate, up, sub_w, h_out, nullptr, hq))
+        return rows_relu2_norm_quant(static_cast<const __half*>(gate), static_cast<const __half*>(up), sub_w,
+                                     static_cast<__half*>(h_out), hq, d_absmax, n, eps, stream, vectors);
     const size_t smem = sizeof(float) * static_cast<size_t>(n);
     if (smem > 200 * 1024) return fail(SPB_E_UNSUPPORTED, "relu2_norm_quant: n=%d too large", n);
     if (smem > 48 * 1024) cudaFuncSetAttribute(relu2_norm_quant_kernel,
@@ -389,6 +396,10 @@ int relu2_norm_quant(const void* gate, const void* up, const float* sub_w, void*
 int rope_scatter(void* q, const void* k, const void* v, void* kcache, void* vcache, int num_heads,
                  int num_kv_heads, int head_dim, int max_seq_len, float theta, const int* d_pos,
                  void* stream, int vectors, size_t seq_stride) {
+    if (rows_rope_scatter_takes(q, k, v, kcache, vcache, head_dim, seq_stride))
+        return rows_rope_scatter(static_cast<__half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
+                                 static_cast<__half*>(kcache), static_cast<__half*>(vcache), num_heads, num_kv_heads, head_dim,
+                                 max_seq_len, theta, d_pos, stream, vectors, seq_stride);
     const int threads = (num_heads + num_kv_heads) * (head_dim / 2) + num_kv_heads * head_dim / 2;
     return launch("rope_scatter", rope_scatter_kernel, dim3((threads + 255) / 256, vectors), dim3(256), 0, stream,
                   static_cast<__half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),

@@ -5,6 +5,7 @@
 //   absmax_quantize_rows : absmax_quantize_gpu (src/kernels/inference_kernels.cu:69-114) per row
 //   dequantize_rows      : dequantize_gpu (src/kernels/inference_kernels.cu:162-171) per row, each row with its own absmax
 #include "fused_ops.cuh"
+#include "row_ops.cuh"
 
 namespace spb {
 
@@ -87,6 +88,8 @@ int embed_rows(const void* embed, const int* d_tokens, void* x, int hidden, int 
 }
 
 int absmax_quantize_rows(const void* in, int8_t* out, float* d_absmax, int n, int vectors, void* stream) {
+    if (row_ops_take(n, in, nullptr, nullptr, nullptr, nullptr, out))
+        return rows_absmax_quantize(static_cast<const __half*>(in), out, d_absmax, n, stream, vectors);
     int t = ((n + 3) / 4 + 31) & ~31;
     t = max(32, min(1024, t));
     return launch("absmax_quantize_rows", absmax_quantize_rows_kernel, dim3(vectors), dim3(t), 0, stream,
