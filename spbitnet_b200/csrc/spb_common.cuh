@@ -70,6 +70,30 @@ int launch(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return SPB_OK;
 }
 
+// launch() with thread-block clusters of `cluster` blocks along x
+template <typename... KArgs, typename... Args>
+int launch_clustered(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, void* stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SPB_E_CUDA, "%s: launch failed: %s", name, cudaGetErrorString(err));
+    }
+    return SPB_OK;
+}
+
 // griddepcontrol.launch_dependents: lets the next grid on the stream begin its independent prologue
 // (weight prefetch).  Harmless without PDL.  Most kernels call it first thing; the tensor-core GEMV
 // calls it after its own dependency wait, which keeps at most one waiting grid per stream resident
