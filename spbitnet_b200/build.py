@@ -18,7 +18,7 @@ LIB = HERE / "libspbitnet_b200.so"
 CLI = HERE / "spbitnet_infer"
 CALLS = HERE / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["core.cu", "gemv.cu", "gemv_batch_mma.cu", "gemv_mmasp.cu", "gemv_prepared.cu", "gemm.cu", "gemm_tcsp_ws.cu", "half_gemm_tc.cu", "gemm_mmasp.cu", "unpack.cu",
-           "decode_ops.cu", "attention.cu", "attention_prefill.cu", "fused_ops.cu", "row_ops.cu", "prefill.cu", "decode_persistent.cu", "engine.cu", "sharded.cu", "noalloc.cu", "pack.cu", "format_host.cpp",
+           "decode_ops.cu", "attention.cu", "attention_prefill.cu", "attention_batch.cu", "fused_ops.cu", "row_ops.cu", "prefill.cu", "decode_persistent.cu", "engine.cu", "sharded.cu", "noalloc.cu", "pack.cu", "format_host.cpp",
            "tokenizer.cpp", "model_loader.cpp"]
 COMPILE_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
                  "-Xcompiler", "-fPIC"]

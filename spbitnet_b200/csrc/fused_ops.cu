@@ -410,6 +410,8 @@ int rope_scatter(void* q, const void* k, const void* v, void* kcache, void* vcac
 int decode_attention_pos(const void* Q, const void* K, const void* V, void* out, int num_heads,
                          int num_kv_heads, int head_dim, int max_seq_len, float scale, const int* d_pos,
                          void* stream, int vectors, size_t seq_stride) {
+    if (batch_attention_supported(K, V, out, num_heads, num_kv_heads, head_dim, seq_stride))
+        return batch_attention(Q, K, V, out, num_heads, num_kv_heads, head_dim, max_seq_len, scale, d_pos, stream, vectors, seq_stride);
     const size_t smem = sizeof(float) * (((max_seq_len + 31) & ~31) + 8 * static_cast<size_t>(head_dim));
     if (smem > 200 * 1024) return fail(SPB_E_UNSUPPORTED, "decode_attention: max_seq_len %d too long", max_seq_len);
     if (smem > 48 * 1024) cudaFuncSetAttribute(decode_attention_pos_kernel,

@@ -45,6 +45,11 @@ int decode_attention_pos(const void* Q, const void* K, const void* V, void* out,
 int prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads, int num_kv_heads,
                       int head_dim, int max_seq_len, float scale, const int* d_pos, void* stream);
 bool prefill_attention_supported(int num_heads, int num_kv_heads, int head_dim);
+// attention_batch.cu: what decode_attention_pos runs on for many vectors where the shape allows it
+bool batch_attention_supported(const void* K, const void* V, const void* out, int num_heads, int num_kv_heads, int head_dim,
+                               size_t seq_stride);
+int batch_attention(const void* Q, const void* K, const void* V, void* out, int num_heads, int num_kv_heads, int head_dim,
+                    int max_seq_len, float scale, const int* d_pos, void* stream, int vectors, size_t seq_stride);
 // attention.cu: split-KV decode attention.  seq_len comes from *d_pos + 1 when d_pos is given.
 // `counters` (optional): num_kv_heads zeroed words; with them the merge of a KV head's chunks runs inside the same
 // launch, in the block that finishes last, instead of as a second kernel.  They are left at zero.
