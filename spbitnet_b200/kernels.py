@@ -246,8 +246,8 @@ def prune_pack_gpu(weights, stream=None):
     assert weights.is_cuda and weights.dtype == torch.float32 and weights.dim() == 2 and weights.stride(1) == 1
     rows, cols = weights.shape
     ms, vs = (cols // 4 + 7) // 8, (cols // 4 + 15) // 16
-    meta = torch.zeros((rows, ms), dtype=torch.int32, device=weights.device)
-    values = torch.zeros((rows, vs), dtype=torch.int32, device=weights.device)
+    meta = torch.empty((rows, ms), dtype=torch.int32, device=weights.device)  # every word of the tight rows is written
+    values = torch.empty((rows, vs), dtype=torch.int32, device=weights.device)
     abs_sum = torch.zeros(1, dtype=torch.float64, device=weights.device)
     _c.spb_prune_pack_gpu(weights, rows, cols, weights.stride(0), meta, values, ms, vs, abs_sum, stream)
     gamma = float(abs_sum.item()) / max(1, rows * cols)

@@ -81,3 +81,36 @@ def test_strided_input_and_bad_arguments():
     assert lib.spb_prune_pack_gpu(big.data_ptr(), 8, 302, 302, big.data_ptr(), big.data_ptr(), 10, 5, None, None) != 0
     assert lib.spb_prune_pack_gpu(big.data_ptr(), 8, 256, 300, big.data_ptr(), big.data_ptr(), 7, 4, None, None) != 0
     assert lib.spb_prune_pack_gpu(big.data_ptr(), 0, 256, 300, None, None, 8, 4, None, None) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(5, 1028), (1000, 4), (2, 65536), (33, 260), (700, 64), (4099, 192)])
+def test_units_and_their_remainders(rows, cols):
+    # units of 64 columns, sixteen per warp, rows that end inside one, more units than one pass of the grid takes
+    wf = (np.random.default_rng(cols).standard_normal((rows, cols)) * 0.02).astype(np.float32)
+    meta, values, gamma = run(wf)
+    wm, wv, _ = converter_steps(wf)
+    assert (meta == wm).all() and (values == wv).all()
+    want = np.abs(wf.astype(np.float64)).mean()
+    assert abs(gamma - want) <= 1e-12 * want
+
+
+def test_infinities_and_nans():
+    # kept = at least two of the others sort before it by comparisons of |w|: a NaN compares with nothing
+    rng = np.random.default_rng(3)
+    wf = rng.standard_normal((40, 260)).astype(np.float32)
+    wf[rng.random(wf.shape) < 0.1] = np.inf
+    wf[rng.random(wf.shape) < 0.1] = -np.inf
+    wf[20:][rng.random((20, 260)) < 0.05] = np.nan
+    meta, values, _ = run(wf)
+    a = np.abs(wf).reshape(40, 65, 4)
+    neg = (wf < 0).reshape(40, 65, 4)
+    for r in range(40):
+        for g in range(65):
+            bm = sg = seen = 0
+            for i in range(4):
+                if sum(a[r, g, j] < a[r, g, i] or (a[r, g, j] == a[r, g, i] and j < i) for j in range(4)) >= 2:
+                    bm |= 1 << i
+                    sg |= int(neg[r, g, i]) << seen
+                    seen += 1
+            assert (int(meta[r, g // 8]) >> (4 * (g % 8))) & 15 == bm
+            assert (int(values[r, g // 16]) >> (2 * (g % 16))) & 3 == sg
