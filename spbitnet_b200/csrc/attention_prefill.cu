@@ -8,9 +8,12 @@
 // Tiles of positions start at multiples of 64 whatever the chunk, and a tile past a row's own position leaves the row
 // untouched, so a row's bits do not depend on how a prompt is cut into calls.
 //
-// Bound: the tensor pipe (three products of 16 x 64 x head_dim per warp and tile); a block per (head, token) that walks
-// the positions serially, used before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens
-// at 20 heads of 128, this kernel 73 us.
+// Bound: 20 heads of 128 over 1800 positions keep the tensor pipe busy for half of the active cycles and the chip active for
+// 70 % of them (245 blocks of unequal length on 148 SMs).  A block per (head, token) that walks the positions serially, used
+// before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens; this kernel 73 us, and 62 us since
+// full tiles are not masked, a factor of one is not multiplied into the output and the weights are split two at a time.
+// Two warps per 16 tokens (32 of a tile's positions each) and clusters of two blocks per 16 tokens (alternate tiles) measured
+// the same or slower.
 #include "fused_ops.cuh"
 
 namespace spb {
@@ -34,8 +37,20 @@ __device__ __forceinline__ void pa_mma(float (&d)[4], const uint32_t (&a)[4], ui
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t pa_pack(__half lo, __half hi) {
-    return static_cast<uint32_t>(__half_as_ushort(lo)) | (static_cast<uint32_t>(__half_as_ushort(hi)) << 16);
+// 2^x for x <= 0.  Like exp2f but for results below 2^-126, which come out as zero: next to the row's largest weight, 1, they
+// are below every bit of the sums.
+__device__ __forceinline__ float pa_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// two weights as halves and the halves of what those miss
+__device__ __forceinline__ void pa_split(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
 template <int HD>
@@ -121,13 +136,20 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                     pa_mma(s[2 * nb + 1], qf[k], b[2], b[3]);
                 }
             float na = ma, nb_ = mb;
+            if ((j + 1) * kPaTile - 1 > start + tok0) {  // some of the tile's positions are past some of the warp's rows
+#pragma unroll
+                for (int i = 0; i < kPaTile / 8; ++i) {
+                    const int p = j * kPaTile + i * 8 + 2 * t4;
+                    if (p > pa) s[i][0] = -INFINITY;
+                    if (p + 1 > pa) s[i][1] = -INFINITY;
+                    if (p > pb) s[i][2] = -INFINITY;
+                    if (p + 1 > pb) s[i][3] = -INFINITY;
+                }
+            }
 #pragma unroll
             for (int i = 0; i < kPaTile / 8; ++i) {
-                const int p = j * kPaTile + i * 8 + 2 * t4;
-                s[i][0] = p <= pa ? s[i][0] * scale_log2 : -INFINITY;
-                s[i][1] = p + 1 <= pa ? s[i][1] * scale_log2 : -INFINITY;
-                s[i][2] = p <= pb ? s[i][2] * scale_log2 : -INFINITY;
-                s[i][3] = p + 1 <= pb ? s[i][3] * scale_log2 : -INFINITY;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[i][c] *= scale_log2;
                 na = fmaxf(na, fmaxf(s[i][0], s[i][1]));
                 nb_ = fmaxf(nb_, fmaxf(s[i][2], s[i][3]));
             }
@@ -136,18 +158,21 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                 na = fmaxf(na, __shfl_xor_sync(0xFFFFFFFFu, na, off));
                 nb_ = fmaxf(nb_, __shfl_xor_sync(0xFFFFFFFFu, nb_, off));
             }
-            // position 0 is visible to every row, so the maxima are finite from the first tile on
-            const float ca = exp2f(ma - na), cb = exp2f(mb - nb_);
-            ma = na;
-            mb = nb_;
-            la *= ca;
-            lb *= cb;
+            // position 0 is visible to every row, so the maxima are finite from the first tile on; past the first few tiles
+            // they rarely move, and a factor of one is not multiplied
+            if (__any_sync(0xFFFFFFFFu, !(na == ma && nb_ == mb))) {
+                const float ca = exp2f(ma - na), cb = exp2f(mb - nb_);
+                ma = na;
+                mb = nb_;
+                la *= ca;
+                lb *= cb;
 #pragma unroll
-            for (int i = 0; i < HD / 8; ++i) {
-                o[i][0] *= ca;
-                o[i][1] *= ca;
-                o[i][2] *= cb;
-                o[i][3] *= cb;
+                for (int i = 0; i < HD / 8; ++i) {
+                    o[i][0] *= ca;
+                    o[i][1] *= ca;
+                    o[i][2] *= cb;
+                    o[i][3] *= cb;
+                }
             }
 #pragma unroll
             for (int kk = 0; kk < kPaTile / 16; ++kk) {
@@ -155,22 +180,14 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float* e = s[2 * kk + h];
-                    e[0] = exp2f(e[0] - ma);
-                    e[1] = exp2f(e[1] - ma);
-                    e[2] = exp2f(e[2] - mb);
-                    e[3] = exp2f(e[3] - mb);
+                    e[0] = pa_exp2(e[0] - ma);
+                    e[1] = pa_exp2(e[1] - ma);
+                    e[2] = pa_exp2(e[2] - mb);
+                    e[3] = pa_exp2(e[3] - mb);
                     la += e[0] + e[1];
                     lb += e[2] + e[3];
-                    __half hh[4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        hh[c] = __float2half_rn(e[c]);
-                        e[c] -= __half2float(hh[c]);
-                    }
-                    hi[2 * h] = pa_pack(hh[0], hh[1]);
-                    hi[2 * h + 1] = pa_pack(hh[2], hh[3]);
-                    lo[2 * h] = pa_pack(__float2half_rn(e[0]), __float2half_rn(e[1]));
-                    lo[2 * h + 1] = pa_pack(__float2half_rn(e[2]), __float2half_rn(e[3]));
+                    pa_split(e[0], e[1], hi[2 * h], lo[2 * h]);
+                    pa_split(e[2], e[3], hi[2 * h + 1], lo[2 * h + 1]);
                 }
 #pragma unroll
                 for (int nb = 0; nb < HD / 16; ++nb) {
