@@ -10,7 +10,7 @@
 //
 // Bound: 20 heads of 128 over 1800 positions keep the tensor pipe busy for half of the active cycles and the chip active for
 // 70 % of them (245 blocks of unequal length on 148 SMs).  A block per (head, token) that walks the positions serially, used
-// before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens; this kernel 73 us, and 62 us since
+// before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens; this kernel 75 us, and 66 us since
 // full tiles are not masked, a factor of one is not multiplied into the output and the weights are split two at a time.
 // Two warps per 16 tokens (32 of a tile's positions each) and clusters of two blocks per 16 tokens (alternate tiles) measured
 // the same or slower.
