@@ -79,6 +79,7 @@ struct spb_engine {
     uint2* d_pd_ll = nullptr;         // tagged words of the barrier-free form (decode mode 4)
     size_t pd_ll_words = 0;
     int seq_len = 0;
+    int kv_reached = 0;     // no position from here on has been written since the last reset
     int timeouts_seen = 0;  // value of the library's bounded-wait counter when the engine last looked
 
     // batched prefill: buffers for `pf_cap` tokens at a time, allocated by the first call that needs them
@@ -533,9 +534,14 @@ int run_prefill_chunk(spb_engine* e, int T, bool last) {
     return SPB_OK;
 }
 
+// To be called before n more positions are enqueued (counted from whichever is larger: what failed half-way may have
+// written more than seq_len says).
+void reach(spb_engine* e, int n) { e->kv_reached = std::min(std::max(e->kv_reached, e->seq_len) + n, e->cfg.max_position_embeddings); }
+
 // Runs tokens[0..n) (HOST array) through the model from position e->seq_len in chunks; leaves the logits of
 // the last one in e->logits, *d_pos = e->seq_len = old + n.  Validated by the caller.
 int prefill_tokens(spb_engine* e, const int* tokens, int n) {
+    reach(e, n);
     const int chunk = std::min(e->prefill_chunk > 0 ? e->prefill_chunk : kPrefillMaxChunk, kPrefillMaxChunk);
     int rc = ensure_prefill_buffers(e, std::min(chunk, std::max(n, 1)));
     if (rc) return rc;
@@ -694,6 +700,7 @@ extern "C" int spb_engine_forward(spb_engine* e, int token_id, const float** d_l
     SPB_ON_ENGINE_DEVICE(e);
     if ((rc = ensure_graph(e, false, 0))) return rc;
     if ((rc = set_int(e->d_next, token_id, e->stream))) return rc;
+    reach(e, 1);
     SPB_CUDA(cudaGraphLaunch(e->graph, e->stream));
     e->seq_len++;
     if (d_logits) {
@@ -734,9 +741,10 @@ extern "C" int spb_engine_set_prefill_chunk(spb_engine* e, int chunk) {
 extern "C" int spb_engine_reset(spb_engine* e) {
     if (!e) return fail(SPB_E_INVALID, "spb_engine_reset: null handle");
     SPB_ON_ENGINE_DEVICE(e);
-    const size_t kv_total = e->kv_bytes_per_layer * e->cfg.num_hidden_layers;
-    SPB_CUDA(cudaMemsetAsync(e->kcache, 0, kv_total, e->stream));
-    SPB_CUDA(cudaMemsetAsync(e->vcache, 0, kv_total, e->stream));
+    const spb_model_config& c = e->cfg;
+    for (__half* cache : {e->kcache, e->vcache})
+        SPB_CUDA(clear_cache_positions(cache, c.num_hidden_layers, e->kv_bytes_per_layer, c.num_key_value_heads,
+                                       c.max_position_embeddings, sizeof(__half) * c.head_dim, e->kv_reached, e->stream));
     SPB_CUDA(cudaMemsetAsync(e->d_pos, 0, 16, e->stream));
     // barrier words of the persistent step: a launch that gave up at a barrier leaves them marked broken
     if (e->d_pd_sync)
@@ -745,6 +753,7 @@ extern "C" int spb_engine_reset(spb_engine* e) {
     if (e->d_pd_ll) SPB_CUDA(cudaMemsetAsync(e->d_pd_ll, 0, sizeof(uint2) * e->pd_ll_words, e->stream));
     SPB_CUDA(cudaStreamSynchronize(e->stream));
     e->seq_len = 0;
+    e->kv_reached = 0;
     return SPB_OK;
 }
 
@@ -822,6 +831,7 @@ static int generate_impl(spb_engine* e, const int* prompt, int n_prompt, int max
     }
     SPB_CUDA(cudaMemcpyAsync(e->d_prompt + start, prompt, sizeof(int) * n_prompt, cudaMemcpyHostToDevice, e->stream));
     if ((rc = ensure_graph(e, true, need))) return rc;
+    reach(e, steps);
     int produced = 0;
     if (e->prefill_chunk > 0 && n_prompt >= 2) {
         // The prompt as a batch; the first generated token comes from its last logits, the rest from the

@@ -94,6 +94,11 @@ int launch_clustered(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3
     return SPB_OK;
 }
 
+// Clears positions 0 .. positions - 1 of a cache of `layers` x `rows` runs of max_positions * row_bytes, layers layer_bytes
+// apart, on `stream` (core.cu).
+cudaError_t clear_cache_positions(void* cache, int layers, size_t layer_bytes, size_t rows, int max_positions, size_t row_bytes,
+                                  int positions, cudaStream_t stream);
+
 // griddepcontrol.launch_dependents: lets the next grid on the stream begin its independent prologue
 // (weight prefetch).  Harmless without PDL.  Most kernels call it first thing; the tensor-core GEMV
 // calls it after its own dependency wait, which keeps at most one waiting grid per stream resident
