@@ -691,7 +691,11 @@ extern "C" int spb_engine_set_linear(spb_engine* e, int layer, int which, const 
                     which, rows, cols, want_rows[which], want_cols[which]);
     Linear& L = e->layers[layer].lin[which];
     drop_graph(e);
-    L.prep = nullptr;  // a copy of the tensor this one replaces; its slot is written again, in stream order, when next needed
+    if (L.prep) {  // a copy of the tensor this one replaces, perhaps still being read
+        SPB_ON_ENGINE_DEVICE(e);
+        SPB_CUDA(cudaStreamSynchronize(e->stream));
+        L.prep = nullptr;
+    }
     L.meta = d_meta; L.values = d_values; L.gamma = gamma; L.rows = rows; L.cols = cols;
     L.ms = meta_stride; L.vs = values_stride;
     return SPB_OK;

@@ -84,6 +84,7 @@ __device__ __forceinline__ uint32_t gp_index_pairs(uint32_t m) {
 __global__ void __launch_bounds__(256) gemv_prepare_kernel(const uint32_t* __restrict__ meta, const uint32_t* __restrict__ values,
                                                            int rows, int cols, int meta_stride, int values_stride, int ntiles,
                                                            int nquads, uint8_t* __restrict__ prep) {
+    grid_dep_wait();  // a product that is still running may read the copy that this rewrites; it lets its successors in early
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= static_cast<long long>(ntiles) * nquads * 32) return;
     const int lane = static_cast<int>(i & 31);
