@@ -26,12 +26,15 @@
 // themselves: 21 instructions, no table.
 //
 // LAYOUT = kTiled: cols % 16 == 0, row strides multiples of 4 words, 16-byte aligned meta / values / X (tensor maps).
+// LAYOUT = kSigns8: the same, but sign rows on 8-byte boundaries only, in whole 8-byte pieces: a width that is an odd multiple
+//   of 128 has tight sign rows of 8 (mod 16) bytes, which no tensor map takes.  Warp 18 brings the signs by 8-byte asynchronous
+//   copies, four lanes per row and chunk, on the barrier that the bitmaps' copy completes.  28672 x 5504, n = 200: 27 us, in the
+//   form for any layout 217;  6912 x 3200, n = 64: 9.1 and 17.5;  5000 x 1408, n = 200: 7.5 and 17.1.
 // LAYOUT = kAny: any other: the re-encoding warps load their words themselves, eight warps copy the activation tiles.
 //
 // Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run out of their own
 // bounds, the copy warps wait (bounded) for their copies in flight, tensor memory is freed and the block returns.
 #include <cmath>
-#include <cstring>
 
 #include "gemm_tcsp_ws.cuh"
 #include "tcgen05_ops.cuh"
@@ -51,7 +54,7 @@ constexpr int kWsMaxRing = 8;
 constexpr int kWsBarBytes = 512, kWsScaleBytes = 1024;
 constexpr int kWsSmemCap = 226 * 1024;
 
-enum WsLayout { kTiled = 0, kAny = 1 };
+enum WsLayout { kTiled = 0, kAny = 1, kSigns8 = 2 };
 
 struct WsMat {
     const uint32_t* meta;
@@ -133,8 +136,9 @@ __device__ __forceinline__ void ws_sign_bytes(uint32_t v, uint32_t (&w)[8]) {
 }
 
 template <bool HALF_OUT, int LAYOUT>
-__global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThreadsAny, 1)
+__global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsAny, 1)
     gemm_tcsp_ws_kernel(const WsArgs a, const __grid_constant__ WsMaps maps) {
+    constexpr bool kMapped = LAYOUT != kAny, kAsyncSigns = LAYOUT == kSigns8;
     extern __shared__ uint8_t ws_raw[];
     // [barriers][row scales] ... 1024-aligned: [A ring][activation ring][packed-word ring]; the epilogue's sums take the
     // place of the rings when the products are done
@@ -162,27 +166,48 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
 
     grid_dep_launch();
     const int nchunks = (nsteps + 1) >> 1;
-    auto load_chunk = [&](int c, int s) {  // packed words of 512 columns: 16 words of meta and 8 of values per row
-        const uint32_t bar = w_full + 8 * s, dst = wring_s + s * w_bytes;
+    // packed words of 512 columns, 16 words of meta and 8 of values per row: called by lane 0, with kAsyncSigns by the warp
+    auto load_chunk = [&](int c, int s) {
+        const uint32_t bar = w_full + 8 * s, dst = wring_s + s * w_bytes, vdst = dst + a.mh * kWsTileM * 64;
         const int k2 = s0 + 2 * c;
-        ws_expect(bar, w_bytes);
-        ws_tma(dst, &maps.meta[mi], 8 * k2, row0, bar);
-        ws_tma(dst + a.mh * kWsTileM * 64, &maps.values[mi], 4 * k2, row0, bar);
-    };
-    if (LAYOUT == kTiled && tid == 32 * kWsWWarp) {  // the first chunks leave before the block has set itself up (1100 clocks)
-        for (int s = 0; s < a.sw; ++s) {
-            ws_init(w_full + 8 * s, 1);
-            ws_init(w_free + 8 * s, kWsExpandWarps);
+        if (!kAsyncSigns || lane == 0) {
+            ws_expect(bar, kAsyncSigns ? a.mh * kWsTileM * 64 : w_bytes);
+            ws_tma(dst, &maps.meta[mi], 8 * k2, row0, bar);
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int s = 0; s < min(a.sw, nchunks); ++s) load_chunk(s, s);
+        if (!kAsyncSigns) {
+            ws_tma(vdst, &maps.values[mi], 4 * k2, row0, bar);
+            return;
+        }
+        const int piece = lane & 3, word = 4 * k2 + 2 * piece;  // a lane's two words of every eighth row
+        const bool in_row = word < (a.cols >> 6);
+        for (int r = lane >> 2; r < a.mh * kWsTileM; r += 8) {  // the tensor map's order: 16-byte halves swapped by bit 2 of the row
+            const bool valid = in_row && row0 + r < m.rows;
+            const uint32_t* src = m.values + (valid ? static_cast<size_t>(row0 + r) * m.values_stride + word : 0);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                             vdst + r * 32 + (((piece >> 1) ^ ((r >> 2) & 1)) << 4) + 8 * (piece & 1)),
+                         "l"(src), "r"(valid ? 8 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+    };
+    if (kMapped && warp == kWsWWarp) {  // the first chunks leave before the block has set itself up (1100 clocks)
+        if (lane == 0) {
+            for (int s = 0; s < a.sw; ++s) {
+                ws_init(w_full + 8 * s, kAsyncSigns ? 33 : 1);
+                ws_init(w_free + 8 * s, kWsExpandWarps);
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+        if (kAsyncSigns || lane == 0)
+            for (int s = 0; s < min(a.sw, nchunks); ++s) load_chunk(s, s);
     }
     if (tid == 32 * kWsXWarp) {
-        if (LAYOUT == kTiled) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
+        if (kMapped) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
         for (int s = 0; s < kWsMaxRing; ++s) {
             ws_init(a_full + 8 * s, 8 * a.mh);
             ws_init(a_free + 8 * s, 1);
-            ws_init(b_full + 8 * s, LAYOUT == kTiled ? 1 : kWsCopyWarps);
+            ws_init(b_full + 8 * s, kMapped ? 1 : kWsCopyWarps);
             ws_init(b_free + 8 * s, 1);
         }
         ws_init(done_b, 1);
@@ -201,9 +226,9 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
     const uint32_t tmem_e = tmem_d + static_cast<uint32_t>(a.nt * a.mh);  // metadata slots behind the accumulators
     bool ok = true;
 
-    if (LAYOUT == kTiled && warp == kWsWWarp) {
+    if (kMapped && warp == kWsWWarp) {
         // ---- packed weights: 512 columns of every row per chunk ---------------------------------------------------
-        if (lane == 0) {
+        if (kAsyncSigns || lane == 0) {
             WsCursor w;
             int issued = min(a.sw, nchunks);
             w.ph = 1;
@@ -213,9 +238,10 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
             }
             for (int c = max(0, issued - a.sw); c < issued; ++c)  // nothing in flight when the block leaves
                 if (!ws_wait(w_full + 8 * (c % a.sw), static_cast<uint32_t>(c / a.sw) & 1u, a.wait_cycles)) ok = false;
+            if (kAsyncSigns) asm volatile("cp.async.wait_all;" ::: "memory");
             if (!ok) ws_count_timeout(a.timeouts);
         }
-    } else if (LAYOUT == kTiled && warp == kWsXWarp) {
+    } else if (kMapped && warp == kWsXWarp) {
         // ---- activation tiles ----------------------------------------------------------------------------------------
         if (lane == 0) {
             grid_dep_wait();  // X may be a predecessor's output
@@ -230,7 +256,7 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
                 if (!ws_wait(b_full + 8 * (h % a.sb), static_cast<uint32_t>(h / a.sb) & 1u, a.wait_cycles)) ok = false;
             if (!ok) ws_count_timeout(a.timeouts);
         }
-    } else if (LAYOUT == kAny && warp >= kWsXWarp) {
+    } else if (!kMapped && warp >= kWsXWarp) {
         // ---- activation tiles, any alignment: a warp per batch row and half step, four columns per lane ------------
         grid_dep_wait();
         const int cw = warp - kWsXWarp;
@@ -350,9 +376,9 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
         ca.s = first;  // fewer steps than stages ahead: first < sa
         uint4 mm, mn;
         uint2 vv, vn;
-        if (LAYOUT == kAny) load_words(first, mn, vn);
+        if (!kMapped) load_words(first, mn, vn);
         for (int i = first; i < nsteps; i += stride, ca.advance(a.sa, stride)) {
-            if (LAYOUT == kTiled) {
+            if (kMapped) {
                 const int s = cw.s, x = i & 1;
                 ok = ws_wait(w_full + 8 * s, cw.ph, a.wait_cycles);
                 ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
@@ -400,7 +426,7 @@ __global__ void __launch_bounds__(LAYOUT == kTiled ? kWsThreadsTiled : kWsThread
             if (lane == 0) ws_arrive(a_full + 8 * sA);
             // The chunk is given back only here, after its words have gone through registers into the stores above: with the
             // arrival right behind the loads the copy engine overwrote words that a load still had to read.
-            if (LAYOUT == kTiled && (a.mh == 1 || (i & 1))) {
+            if (kMapped && (a.mh == 1 || (i & 1))) {
                 if (lane == 0) ws_arrive(w_free + 8 * cw.s);
                 cw.advance(a.sw);
             }
@@ -645,26 +671,29 @@ static WsShape ws_choose(const TcspMat* mats, int nmat, int cols, int n, bool ti
 int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const float* absmax, int cols, int n, void* stream) {
     const char* name = "spb_sparse_ternary_gemm(tcgen05.sp)";
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    bool tiled = cols % 16 == 0 && al(X);
-    for (int i = 0; i < nmat; ++i)
-        tiled = tiled && al(mats[i].meta) && al(mats[i].values) && mats[i].meta_stride % 4 == 0 && mats[i].values_stride % 4 == 0;
+    bool tiled = cols % 16 == 0 && al(X), signs16 = true, signs8 = cols % 128 == 0;
+    for (int i = 0; i < nmat; ++i) {
+        tiled = tiled && al(mats[i].meta) && mats[i].meta_stride % 4 == 0;
+        signs16 = signs16 && al(mats[i].values) && mats[i].values_stride % 4 == 0;
+        signs8 = signs8 && (reinterpret_cast<uintptr_t>(mats[i].values) & 7u) == 0 && mats[i].values_stride % 2 == 0;
+    }
+    tiled = tiled && (signs16 || signs8);
     WsArgs a{};
-    alignas(64) WsMaps maps;
+    alignas(64) WsMaps maps{};
     WsShape c = ws_choose(mats, nmat, cols, n, tiled);
     auto encode_all = [&] {
         bool good = ws_map(&maps.x, CU_TENSOR_MAP_DATA_TYPE_UINT8, X, cols, n, cols, 128, c.nt, CU_TENSOR_MAP_SWIZZLE_128B);
         for (int i = 0; i < nmat && good; ++i)
             good = ws_map(&maps.meta[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, mats[i].meta, (cols + 31) / 32, mats[i].rows,
                           static_cast<size_t>(mats[i].meta_stride) * 4, 16, c.mh * kWsTileM, CU_TENSOR_MAP_SWIZZLE_64B) &&
-                   ws_map(&maps.values[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, mats[i].values, (cols + 63) / 64, mats[i].rows,
-                          static_cast<size_t>(mats[i].values_stride) * 4, 8, c.mh * kWsTileM, CU_TENSOR_MAP_SWIZZLE_32B);
+                   (!signs16 || ws_map(&maps.values[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, mats[i].values, (cols + 63) / 64, mats[i].rows,
+                          static_cast<size_t>(mats[i].values_stride) * 4, 8, c.mh * kWsTileM, CU_TENSOR_MAP_SWIZZLE_32B));
         return good;
     };
     if (tiled && !encode_all()) {
         tiled = false;
         c = ws_choose(mats, nmat, cols, n, tiled);
     }
-    if (!tiled) memset(&maps, 0, sizeof maps);
     a.X = X;
     a.absmax = absmax;
     a.nmat = nmat;
@@ -687,7 +716,8 @@ int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const fl
     a.timeouts = timeout_counter();
     a.wait_cycles = kWsWaitCycles;
     using Kernel = void (*)(WsArgs, WsMaps);
-    const Kernel kernel = tiled ? (absmax ? gemm_tcsp_ws_kernel<true, kTiled> : gemm_tcsp_ws_kernel<false, kTiled>)
+    const Kernel kernel = tiled && signs16 ? (absmax ? gemm_tcsp_ws_kernel<true, kTiled> : gemm_tcsp_ws_kernel<false, kTiled>)
+                          : tiled          ? (absmax ? gemm_tcsp_ws_kernel<true, kSigns8> : gemm_tcsp_ws_kernel<false, kSigns8>)
                                 : (absmax ? gemm_tcsp_ws_kernel<true, kAny> : gemm_tcsp_ws_kernel<false, kAny>);
     if (int rc = ensure_dynamic_smem(name, kernel, c.smem)) return rc;
     cudaLaunchConfig_t cfg = {};
