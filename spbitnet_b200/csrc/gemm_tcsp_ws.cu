@@ -135,7 +135,8 @@ __device__ __forceinline__ void ws_sign_bytes(uint32_t v, uint32_t (&w)[8]) {
     }
 }
 
-template <bool HALF_OUT, int LAYOUT>
+// ROWS4: every output starts its groups of four rows on a boundary of four elements (rows % 4 == 0, an aligned base)
+template <bool HALF_OUT, int LAYOUT, bool ROWS4>
 __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsAny, 1)
     gemm_tcsp_ws_kernel(const WsArgs a, const __grid_constant__ WsMaps maps) {
     constexpr bool kMapped = LAYOUT != kAny, kAsyncSigns = LAYOUT == kSigns8;
@@ -435,8 +436,11 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
     }
     __syncwarp();
     // ---- epilogue: accumulators -> shared memory, [column][128 rows] words in place of the rings -> output.  Every
-    //      thread of the block then takes four rows of a column: the output is written 256 (512) bytes at a time.  In a
-    //      cluster block z adds and stores the columns [z cs, + cs) of all blocks' sums.
+    //      thread of the block then takes four rows of a column: the output is written 256 (512) bytes at a time.  Where four
+    //      rows do not lie on one boundary that would be four stores of 2 (4) bytes at a stride of 8 (16), so a block that has
+    //      no peers stores from the registers, 32 consecutive rows at a time (1001 x 640, n = 64, int32: 5.2 -> 4.5 us; with
+    //      rows on such boundaries the way through shared memory is the faster one, 28672 x 640, n = 200, half: 10.5
+    //      against 12.5 us).  In a cluster block z adds and stores the columns [z cs, + cs) of all blocks' sums.
     grid_dep_wait();  // the output may still be read by a predecessor, the scales are its result
     if (HALF_OUT && tid < a.nt) scales[tid] = dequant_scale(m.gamma, a.absmax[min(n0 + tid, a.n - 1)]);
     if (warp < kWsExpandWarps) {
@@ -446,21 +450,42 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();  // every copy has landed and every MMA is done (or a wait ran out: the output is unspecified)
-    const bool vec_out = m.rows % 4 == 0 && (reinterpret_cast<uintptr_t>(m.out) & (HALF_OUT ? 7u : 15u)) == 0;
     const int S = a.split, cs = (a.nt + S - 1) / S, me = static_cast<int>(blockIdx.z);
-    for (int g = 0; g < a.mh; ++g) {
-        if (warp < kWsExpandWarps && ok)  // tensor-memory lanes 32 (w % 4) .. + 31, 16 columns at a time
+    auto sums16 = [&](int g, int c0, uint32_t (&r)[16]) {  // tensor-memory lanes 32 (w % 4) .. + 31, 16 columns
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(g * a.nt + c0))
+            : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    };
+    if (!ROWS4 && S == 1 && warp < kWsExpandWarps && ok)
+        for (int g = 0; g < a.mh; ++g) {  // a lane's row, 32 consecutive rows per store
+            const int row = row0 + g * kWsTileM + (warp & 3) * 32 + lane;
             for (int c0 = 16 * (warp >> 2); c0 < a.nt; c0 += 64) {
                 uint32_t r[16];
-                const uint32_t taddr = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(g * a.nt + c0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                sums16(g, c0, r);
+                if (row >= m.rows) continue;
+                const int left = a.n - n0 - c0;  // batch rows of these columns
+                const size_t o = static_cast<size_t>(n0 + c0) * m.rows + row;
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (i < left) {
+                        if (HALF_OUT)
+                            static_cast<__half*>(m.out)[o + static_cast<size_t>(i) * m.rows] =
+                                __float2half_rn(__fmul_rn(static_cast<float>(static_cast<int>(r[i])), scales[c0 + i]));
+                        else
+                            static_cast<int32_t*>(m.out)[o + static_cast<size_t>(i) * m.rows] = static_cast<int>(r[i]);
+                    }
+            }
+        }
+    for (int g = 0; g < (ROWS4 || S > 1 ? a.mh : 0); ++g) {
+        if (warp < kWsExpandWarps && ok)
+            for (int c0 = 16 * (warp >> 2); c0 < a.nt; c0 += 64) {
+                uint32_t r[16];
+                sums16(g, c0, r);
                 const uint32_t at = ring_s + static_cast<uint32_t>((c0 * kWsTileM + (warp & 3) * 32 + lane) * 4);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + i * kWsTileM * 4), "r"(r[i]) : "memory");
@@ -503,7 +528,7 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
                 h[2] = __float2half_rn(__fmul_rn(static_cast<float>(sum.z), sc));
                 h[3] = __float2half_rn(__fmul_rn(static_cast<float>(sum.w), sc));
                 __half* dst = static_cast<__half*>(m.out) + o;
-                if (vec_out) {
+                if (ROWS4) {
                     *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
                 } else {
 #pragma unroll
@@ -512,7 +537,7 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
                 }
             } else {
                 int32_t* dst = static_cast<int32_t*>(m.out) + o;
-                if (vec_out) {
+                if (ROWS4) {
                     *reinterpret_cast<int4*>(dst) = sum;
                 } else {
                     const int32_t v[4] = {sum.x, sum.y, sum.z, sum.w};
@@ -716,9 +741,17 @@ int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const fl
     a.timeouts = timeout_counter();
     a.wait_cycles = kWsWaitCycles;
     using Kernel = void (*)(WsArgs, WsMaps);
-    const Kernel kernel = tiled && signs16 ? (absmax ? gemm_tcsp_ws_kernel<true, kTiled> : gemm_tcsp_ws_kernel<false, kTiled>)
-                          : tiled          ? (absmax ? gemm_tcsp_ws_kernel<true, kSigns8> : gemm_tcsp_ws_kernel<false, kSigns8>)
-                                : (absmax ? gemm_tcsp_ws_kernel<true, kAny> : gemm_tcsp_ws_kernel<false, kAny>);
+    static const Kernel kernels[3][2][2] = {  // layout, half output, four rows on a boundary
+        {{gemm_tcsp_ws_kernel<false, kTiled, false>, gemm_tcsp_ws_kernel<false, kTiled, true>},
+         {gemm_tcsp_ws_kernel<true, kTiled, false>, gemm_tcsp_ws_kernel<true, kTiled, true>}},
+        {{gemm_tcsp_ws_kernel<false, kAny, false>, gemm_tcsp_ws_kernel<false, kAny, true>},
+         {gemm_tcsp_ws_kernel<true, kAny, false>, gemm_tcsp_ws_kernel<true, kAny, true>}},
+        {{gemm_tcsp_ws_kernel<false, kSigns8, false>, gemm_tcsp_ws_kernel<false, kSigns8, true>},
+         {gemm_tcsp_ws_kernel<true, kSigns8, false>, gemm_tcsp_ws_kernel<true, kSigns8, true>}}};
+    bool rows4 = true;
+    for (int i = 0; i < nmat; ++i)
+        rows4 = rows4 && mats[i].rows % 4 == 0 && (reinterpret_cast<uintptr_t>(mats[i].out) & (absmax ? 7u : 15u)) == 0;
+    const Kernel kernel = kernels[!tiled ? kAny : signs16 ? kTiled : kSigns8][absmax != nullptr][rows4];
     if (int rc = ensure_dynamic_smem(name, kernel, c.smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, (n + c.nt - 1) / c.nt, c.split);
