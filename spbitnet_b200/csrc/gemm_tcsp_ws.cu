@@ -34,7 +34,9 @@
 //
 // Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run out of their own
 // bounds, the copy warps wait (bounded) for their copies in flight, tensor memory is freed and the block returns.
+#include <atomic>
 #include <cmath>
+#include <mutex>
 
 #include "gemm_tcsp_ws.cuh"
 #include "tcgen05_ops.cuh"
@@ -605,13 +607,16 @@ static EncodeFn tensor_map_encoder() {
     return encode;
 }
 
+static const int* ws_max_clusters();
+
 // Everything the launchers look up or allocate lazily on the host (driver entry point, the pinned timeout counter,
-// the SM count), done now: an engine calls this at creation so that none of it first happens inside a stream
+// the SM and cluster counts), done now: an engine calls this at creation so that none of it first happens inside a stream
 // capture, where allocations and look-ups are not allowed.
 void prepare_host_state() {
     tensor_map_encoder();
     timeout_counter();
     sm_count();
+    ws_max_clusters();
 }
 
 bool ws_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int inner, int outer,
@@ -649,6 +654,43 @@ static void ws_rings(WsShape& c, bool tiled) {
     c.smem = kWsBarBytes + kWsScaleBytes + 1024 + static_cast<size_t>(max(used(), c.nt * kWsTileM * 4));
 }
 
+constexpr int kWsMaxSplit = 8;
+// Clusters of S = 1 .. kWsMaxSplit blocks, one block per SM, that the current device holds at a time: table[S].  A cluster sits
+// in one GPC, so it is less than SMs / S by an amount that only the driver knows; asked once per device.
+static const int* ws_max_clusters() {
+    static int table[64][kWsMaxSplit + 1];
+    static std::atomic<bool> ready[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (ready[dev].load(std::memory_order_acquire)) return table[dev];
+    std::lock_guard<std::mutex> lock(mu);
+    const auto kernel = gemm_tcsp_ws_kernel<true, kTiled, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kWsThreadsTiled);
+    cfg.dynamicSmemBytes = kWsSmemCap;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool can_ask = ensure_dynamic_smem("cluster occupancy", kernel, cfg.dynamicSmemBytes) == SPB_OK;
+    table[dev][1] = sm_count();
+    for (int S = 2; S <= kWsMaxSplit; ++S) {
+        cfg.gridDim = dim3(1, 1, S);
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = S;
+        int n = 0;
+        if (!can_ask || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = max(1, sm_count() * 3 / 4 / S);
+        }
+        table[dev][S] = n;
+    }
+    ready[dev].store(true, std::memory_order_release);
+    return table[dev];
+}
+
 // How a product is cut: 128- or 256-row blocks, batch rows per block, blocks per cluster along K: the least of
 //   waves * (start + steps * clocks per step + drain [+ exchange])
 // in clocks, as measured (nt = batch rows per block, clocks per step of 256 columns):
@@ -659,7 +701,7 @@ static void ws_rings(WsShape& c, bool tiled) {
 //   drain: 9 per batch row to stage the sums, 16 to write them out;
 //   exchange: two cluster barriers and (S - 1) / S of the sums at 13 B per clock, in place of writing them all out.
 static WsShape ws_choose(const TcspMat* mats, int nmat, int cols, int n, bool tiled) {
-    const int sms = sm_count();
+    const int* clusters = ws_max_clusters();
     const int steps = (cols + kWsStepK - 1) / kWsStepK;
     WsShape best{};
     double best_cost = 1e30;
@@ -674,10 +716,8 @@ static WsShape ws_choose(const TcspMat* mats, int nmat, int cols, int n, bool ti
             if (nt > max_nt || (nn > first && nt < 64)) continue;
             const long long blocks = tiles * ((n + nt - 1) / nt);
             const double step = mh == 2 ? fmax(1250.0, 370.0 + 5.6 * nt) : fmax(690.0, 330.0 + 2.8 * nt);
-            for (int S = 1; S <= (mh == 1 ? 8 : 1) && S <= steps; ++S) {
-                // a cluster sits in one GPC: groups of five to eight leave some of its 18 or so SMs idle
-                const int slots = S <= 2 ? sms : S <= 4 ? sms * 15 / 16 : sms * 7 / 8;
-                const double waves = ceil(static_cast<double>(blocks) * S / slots);
+            for (int S = 1; S <= (mh == 1 ? kWsMaxSplit : 1) && S <= steps; ++S) {
+                const double waves = ceil(static_cast<double>(blocks) / clusters[S]);
                 const double out = S > 1 ? 2800.0 + 36.0 * nt * (S - 1) / S : 16.0 * nt * mh;
                 const double cost = waves * (4500.0 + (steps + S - 1) / S * step + 9.0 * nt * mh + out);
                 if (cost < best_cost) {
