@@ -52,7 +52,6 @@ constexpr int kWsMmaWarp = 16, kWsXWarp = 17, kWsWWarp = 18;
 constexpr int kWsThreadsTiled = 32 * 19;
 constexpr int kWsCopyWarps = 8;                // kAny: warps 17 .. 24 copy the activation tiles
 constexpr int kWsThreadsAny = 32 * (kWsXWarp + kWsCopyWarps);
-constexpr int kWsMaxRing = 8;
 constexpr int kWsBarBytes = 512, kWsScaleBytes = 1024;
 constexpr int kWsSmemCap = 226 * 1024;
 
@@ -207,9 +206,11 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
     }
     if (tid == 32 * kWsXWarp) {
         if (kMapped) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
-        for (int s = 0; s < kWsMaxRing; ++s) {
+        for (int s = 0; s < a.sa; ++s) {
             ws_init(a_full + 8 * s, 8 * a.mh);
             ws_init(a_free + 8 * s, 1);
+        }
+        for (int s = 0; s < a.sb; ++s) {
             ws_init(b_full + 8 * s, kMapped ? 1 : kWsCopyWarps);
             ws_init(b_free + 8 * s, 1);
         }
@@ -711,9 +712,13 @@ static WsShape ws_choose(const TcspMat* mats, int nmat, int cols, int n, bool ti
         for (int i = 0; i < nmat; ++i) tiles += (mats[i].rows + mh * kWsTileM - 1) / (mh * kWsTileM);
         const int max_nt = mh == 2 ? 240 : 256;
         const int first = (n + max_nt - 1) / max_nt;
-        for (int nn = first; nn <= first + 3; ++nn) {
+        // a few cuts of the batch; of short blocks, where start and drain are most of the time, as many as run at once (384 x 640,
+        // n = 900, int32: 5.5 us in blocks of 144 rows, 4.9 in blocks of 64; at six steps or more narrower blocks lose)
+        const int more = steps <= 4 ? clusters[1] : 0;
+        for (int nn = first;; ++nn) {
             const int nt = ((n + nn - 1) / nn + 15) / 16 * 16;
-            if (nt > max_nt || (nn > first && nt < 64)) continue;
+            if (nn > first && (nt < 64 || (nn > first + 3 && tiles * nn > more))) break;
+            if (nt > max_nt) continue;
             const long long blocks = tiles * ((n + nt - 1) / nt);
             const double step = mh == 2 ? fmax(1250.0, 370.0 + 5.6 * nt) : fmax(690.0, 330.0 + 2.8 * nt);
             for (int S = 1; S <= (mh == 1 ? kWsMaxSplit : 1) && S <= steps; ++S) {
