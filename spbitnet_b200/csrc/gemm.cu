@@ -145,18 +145,16 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_generic_kernel(const GemmAr
 // prefill.cu
 int dequantize_rows(const int32_t* acc, void* out, const float* d_absmax, float gamma, int rows, int vectors,
                     void* stream);
-bool gemm_mmasp_supported(const uint32_t* meta, const uint32_t* values, const int8_t* X, int rows, int cols, int n,
-                          int meta_stride, int values_stride, int max_n);
-int gemm_mmasp_launch(const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y, int rows, int cols,
-                      int n, int meta_stride, int values_stride, void* stream, const GemmEpilogue* ep);
 
 // 0 automatic, 1 SIMT form, 3 tcgen05 sparse form, 4 warp-level sparse MMA form where the layout allows it, else 3.
-// Automatic: the warp-level form costs one pass of re-encoding per eight batch rows and starts sooner, so it keeps up to
-// eight rows (6912x2560, n = 8: 4.4 against 6.3 us; n = 16: 6.8 against 6.3; n = 64: 14.9 against 7.0) of matrices up to
-// 40 M weights (8192x8192, n = 8: 12.8 against 11.1 us); the tcgen05 form takes the rest and every layout.
+// Automatic: the warp-level form where it applies and is the faster one (gemm_mmasp_preferred), else the tcgen05 form, which
+// takes every layout.
 static int g_gemm_variant = 0;
-constexpr int kMmaSpAutoMaxN = 8;
-constexpr long long kMmaSpAutoMaxWeights = 40ll << 20;
+// Whether one launch of the warp-level form takes these matrices
+static bool use_mmasp(const TcspMat* mats, int nmat, const int8_t* X, int cols, int n, bool half_out) {
+    return (g_gemm_variant == 4 || (g_gemm_variant == 0 && gemm_mmasp_preferred(mats, nmat, cols, n, half_out))) &&
+           gemm_mmasp_supported(mats, nmat, X, cols, n);
+}
 
 }  // namespace spb
 
@@ -210,18 +208,13 @@ static int gemm_dispatch(const char* name, const uint32_t* meta, const uint32_t*
     auto al = [](const void* p, size_t k) { return (reinterpret_cast<uintptr_t>(p) & (k - 1)) == 0; };
     const bool fast = cols % 128 == 0 && cols / 128 <= 512 && meta_row_stride % 4 == 0 &&
                       values_row_stride % 2 == 0 && al(meta, 16) && al(values, 8) && al(X, 16);
-    const int mma_auto_max_n = static_cast<long long>(rows) * cols <= kMmaSpAutoMaxWeights ? kMmaSpAutoMaxN : 0;
-    if ((g_gemm_variant == 0 || g_gemm_variant == 4) &&
-        gemm_mmasp_supported(meta, values, X, rows, cols, n, meta_row_stride, values_row_stride,
-                             g_gemm_variant == 4 ? 4096 : mma_auto_max_n))
-        return gemm_mmasp_launch(meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream, ep);
-    if (g_gemm_variant != 1 && (fast || !ep || Y)) {
-        // tcgen05 sparse form, any layout.  The scaled output of a layout without 16-byte rows keeps asking for the workspace
-        // that spb_sparse_bitlinear_gemm documents, although this form does not write to it.
-        const TcspMat m{meta, values, ep ? static_cast<void*>(ep->out) : Y, ep ? ep->gamma : 0.0f, rows, meta_row_stride,
-                        values_row_stride};
-        return gemm_tcsp_ws_launch(&m, 1, X, ep ? ep->absmax : nullptr, cols, n, stream);
-    }
+    const TcspMat m{meta, values, ep ? static_cast<void*>(ep->out) : Y, ep ? ep->gamma : 0.0f, rows, meta_row_stride,
+                    values_row_stride};
+    const float* absmax = ep ? ep->absmax : nullptr;
+    if (use_mmasp(&m, 1, X, cols, n, ep != nullptr)) return gemm_mmasp_launch(&m, 1, X, absmax, cols, n, stream);
+    // tcgen05 sparse form, any layout.  The scaled output of a layout without 16-byte rows keeps asking for the workspace that
+    // spb_sparse_bitlinear_gemm documents, although this form does not write to it.
+    if (g_gemm_variant != 1 && (fast || !ep || Y)) return gemm_tcsp_ws_launch(&m, 1, X, absmax, cols, n, stream);
     if (ep) {  // the SIMT forms write int32 sums: run them into the workspace, then scale row by row
         if (!Y) return fail(SPB_E_UNSUPPORTED, "%s: this layout needs acc_workspace (n * rows int32)", name);
         const int rc = gemm_dispatch_int(name, meta, values, X, Y, rows, cols, n, meta_row_stride, values_row_stride, stream,
@@ -234,12 +227,16 @@ static int gemm_dispatch(const char* name, const uint32_t* meta, const uint32_t*
 
 namespace spb {
 
-// BitLinear layers of one width on the same n quantised rows: one launch where the tcgen05 form takes them all (a matrix of
-// five row tiles has no SMs to fill on its own), else one after the other.
+// BitLinear layers of one width on the same n quantised rows: one launch of either form (a matrix of five row tiles has no SMs
+// to fill on its own), else, where it is to be neither of the two, one after the other.  From nine rows on always the tcgen05
+// form: in an engine's chain it has its weights on the way before its turn (prompt of 9 tokens, 24 layers of 2048: 0.98 ms,
+// with the warp-level form for the products that are faster on it by themselves 1.08 ms).
 int bitlinear_gemm_group(const TcspMat* mats, int nmat, const int8_t* Xq, const float* absmax, int cols, int n,
                          int32_t* acc_workspace, void* stream) {
-    const bool one = nmat <= kWsMaxMats && (g_gemm_variant == 3 || (g_gemm_variant == 0 && n > kMmaSpAutoMaxN)) && cols % 4 == 0;
-    if (one) return gemm_tcsp_ws_launch(mats, nmat, Xq, absmax, cols, n, stream);
+    if (nmat <= kWsMaxMats && cols % 4 == 0) {
+        if ((n <= 8 || g_gemm_variant == 4) && use_mmasp(mats, nmat, Xq, cols, n, true)) return gemm_mmasp_launch(mats, nmat, Xq, absmax, cols, n, stream);
+        if (g_gemm_variant != 1) return gemm_tcsp_ws_launch(mats, nmat, Xq, absmax, cols, n, stream);
+    }
     for (int i = 0; i < nmat; ++i)
         if (int rc = spb_sparse_bitlinear_gemm(mats[i].meta, mats[i].values, Xq, mats[i].out, absmax, mats[i].gamma, acc_workspace,
                                                mats[i].rows, cols, n, mats[i].meta_stride, mats[i].values_stride, stream))

@@ -1,6 +1,7 @@
-// Small-batch sparse-ternary product on the warp-level sparse MMA (mma.sp m16n8k64, int8), sm_100a.
+// Small-batch sparse-ternary product on the warp-level sparse MMA (mma.sp m16n8k64, int8), sm_100a, for up to three matrices of
+// one width on the same activation rows (q, k and v of a few prompt tokens, gate and up).
 //
-//   Y[j, r] = sum_c W[r, c] * X[j, c]      W: rows x cols compressed 2:4 ternary, X: n x cols int8, n <= 32
+//   Y[j, r] = sum_c W[r, c] * X[j, c]      W: rows x cols compressed 2:4 ternary, X: n x cols int8, n small
 //
 // The same scheme as the GEMV on this instruction (gemv_mmasp.cu): the raw weight slab of a block comes
 // in by 16-byte asynchronous copies, bitmap words are turned into index pairs and sign nibbles into
@@ -15,7 +16,7 @@
 // as fit in shared memory next to the slab).  Activations are staged after the dependency wait, permuted
 // so that a lane's four B registers of a step are 16 contiguous bytes; row pitch = cols + 64 bytes, which
 // keeps the 16-byte reads of a quarter warp (two activation rows x four lanes) on distinct banks.
-#include "spb_common.cuh"
+#include "gemm_tcsp_ws.cuh"
 
 namespace spb {
 
@@ -24,13 +25,20 @@ constexpr int kGqWarps = kGqThreads / 32;
 constexpr int kGqSignLutBytes = 16 * 32 * 4;  // 2 KB on a 2 KB boundary
 constexpr int kGqMaxTiles = 4;
 
-struct GqArgs {
+struct GqMat {
     const uint32_t* meta;
     const uint32_t* values;
-    const int8_t* X;  // [n, cols]
-    int32_t* Y;       // [n, rows]
-    int rows, cols, n;
-    int meta_stride, values_stride;
+    void* out;  // [n, rows] int32 sums or half
+    float gamma;
+    int rows, meta_stride, values_stride;
+    int blk0;  // first block of this matrix in the grid
+};
+struct GqArgs {
+    GqMat m[kWsMaxMats];
+    int nmat;
+    const int8_t* X;      // [n, cols]
+    const float* absmax;  // row scales of the half outputs
+    int cols, n;
     int steps;    // cols / 64
     int ks;       // warps per row block (power of two <= 8)
     int ks_log2;
@@ -39,7 +47,6 @@ struct GqArgs {
     int mpitch;   // shared-memory row pitch of the bitmap words, in words (= 4 mod 32)
     int vpitch;   // same for the sign words
     int xpitch;   // shared-memory pitch of an activation row, bytes (cols + 64)
-    GemmEpilogue ep;  // ep.out set: scaled half output instead of Y
 };
 
 __device__ __forceinline__ uint32_t gq_index_pairs(uint32_t m) {
@@ -57,7 +64,7 @@ __device__ __forceinline__ uint32_t gq_lds(uint32_t addr) {
 }
 
 // NT = tiles of eight activation rows per block.
-// HALF_OUT: the epilogue writes the scaled half output (a.ep) instead of the int32 sums
+// HALF_OUT: the epilogue writes the scaled half output instead of the int32 sums
 template <int NT, bool HALF_OUT>
 __global__ void __launch_bounds__(kGqThreads, 2) gemm_mmasp_kernel(const GqArgs a) {
     extern __shared__ uint8_t gq_raw[];
@@ -74,8 +81,12 @@ __global__ void __launch_bounds__(kGqThreads, 2) gemm_mmasp_kernel(const GqArgs 
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);  // through a shuffle: known to be uniform over the warp
-    const int row0 = blockIdx.x * nrows_blk;
-    const int valid = min(nrows_blk, a.rows - row0);
+    int mi = 0;
+    if (a.nmat > 1 && static_cast<int>(blockIdx.x) >= a.m[1].blk0) mi = 1;
+    if (a.nmat > 2 && static_cast<int>(blockIdx.x) >= a.m[2].blk0) mi = 2;
+    const GqMat m = mi == 0 ? a.m[0] : mi == 1 ? a.m[1] : a.m[2];
+    const int row0 = (static_cast<int>(blockIdx.x) - m.blk0) * nrows_blk;
+    const int valid = min(nrows_blk, m.rows - row0);
     const int j0 = blockIdx.y * 8 * NT;                       // first activation row of this block
     const uint32_t mbytes = static_cast<uint32_t>(a.cols >> 3), vbytes = static_cast<uint32_t>(a.cols >> 4);
 
@@ -84,9 +95,9 @@ __global__ void __launch_bounds__(kGqThreads, 2) gemm_mmasp_kernel(const GqArgs 
         const int mch = static_cast<int>(mbytes >> 4), cpr = mch + static_cast<int>(vbytes >> 4);
         for (int k = lane; k < cpr; k += 32) {
             const bool is_m = k < mch;
-            const uint8_t* src = is_m ? reinterpret_cast<const uint8_t*>(a.meta) + k * 16
-                                      : reinterpret_cast<const uint8_t*>(a.values) + (k - mch) * 16;
-            const size_t src_pitch = static_cast<size_t>(is_m ? a.meta_stride : a.values_stride) * 4u;
+            const uint8_t* src = is_m ? reinterpret_cast<const uint8_t*>(m.meta) + k * 16
+                                      : reinterpret_cast<const uint8_t*>(m.values) + (k - mch) * 16;
+            const size_t src_pitch = static_cast<size_t>(is_m ? m.meta_stride : m.values_stride) * 4u;
             const uint32_t dst = is_m ? ms_s + static_cast<uint32_t>(k) * 16u : vs_s + static_cast<uint32_t>(k - mch) * 16u;
             const uint32_t dst_pitch = static_cast<uint32_t>(is_m ? a.mpitch : a.vpitch) * 4u;
             src += static_cast<size_t>(row0 + warp) * src_pitch;
@@ -210,34 +221,37 @@ __global__ void __launch_bounds__(kGqThreads, 2) gemm_mmasp_kernel(const GqArgs 
             const int rblk = r >> 4, rr = r & 15;
             int sum = 0;
             for (int k = 0; k < a.ks; ++k) sum += red[(((rblk << a.ks_log2) + k) * 16 + rr) * NC + jc];
-            const size_t o = static_cast<size_t>(j0 + jc) * a.rows + row0 + r;
+            const size_t o = static_cast<size_t>(j0 + jc) * m.rows + row0 + r;
             if (HALF_OUT)
-                a.ep.out[o] = __float2half_rn(__fmul_rn(static_cast<float>(sum), dequant_scale(a.ep.gamma, a.ep.absmax[j0 + jc])));
+                static_cast<__half*>(m.out)[o] = __float2half_rn(__fmul_rn(static_cast<float>(sum), dequant_scale(m.gamma, a.absmax[j0 + jc])));
             else
-                a.Y[o] = sum;
+                static_cast<int32_t*>(m.out)[o] = sum;
         }
     }
 }
 
-// Whether the small-batch form applies: up to max_n activation rows, whole 16-byte sign rows (cols % 256 == 0),
-// 16-byte aligned rows everywhere.
-bool gemm_mmasp_supported(const uint32_t* meta, const uint32_t* values, const int8_t* X, int rows, int cols, int n,
-                          int meta_stride, int values_stride, int max_n) {
+// Whether the form applies: whole 16-byte sign rows (cols % 256 == 0), 16-byte aligned rows everywhere.
+bool gemm_mmasp_supported(const TcspMat* mats, int nmat, const int8_t* X, int cols, int n) {
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    return rows > 0 && n > 0 && n <= max_n && cols > 0 && cols % 256 == 0 && cols <= 16384 &&
-           meta_stride % 4 == 0 && values_stride % 4 == 0 && al16(meta) && al16(values) && al16(X);
+    bool ok = n > 0 && n <= 4096 && cols > 0 && cols % 256 == 0 && cols <= 16384 && al16(X);
+    for (int i = 0; i < nmat; ++i)
+        ok = ok && mats[i].rows > 0 && mats[i].meta_stride % 4 == 0 && mats[i].values_stride % 4 == 0 && al16(mats[i].meta) &&
+             al16(mats[i].values);
+    return ok;
 }
 
-int gemm_mmasp_launch(const uint32_t* meta, const uint32_t* values, const int8_t* X, int32_t* Y, int rows, int cols,
-                      int n, int meta_stride, int values_stride, void* stream, const GemmEpilogue* ep) {
-    const char* name = "spb_sparse_ternary_gemm(mma.sp)";
-    GqArgs a{};
-    a.meta = meta; a.values = values; a.X = X; a.Y = Y;
-    if (ep) a.ep = *ep;
-    a.rows = rows; a.cols = cols; a.n = n;
-    a.meta_stride = meta_stride; a.values_stride = values_stride;
+// Work split and shared memory of a launch: pointers and rows aside, all of GqArgs.
+struct GqShape {
+    int blocks_x, blocks_y, nt;
+    size_t smem;
+};
+static GqShape gq_shape(GqArgs& a, const TcspMat* mats, int nmat, int cols, int n) {
+    a.cols = cols;
+    a.n = n;
+    a.nmat = nmat;
     a.steps = cols / 64;
-    const int row_blocks = (rows + 15) / 16;
+    int row_blocks = 0;
+    for (int i = 0; i < nmat; ++i) row_blocks += (mats[i].rows + 15) / 16;
     a.ks = 8;
     while (a.ks > 1 && a.steps / a.ks < 16) a.ks >>= 1;
     while (a.ks < 8 && row_blocks * a.ks < 2 * sm_count() && a.steps / (2 * a.ks) >= 8) a.ks <<= 1;
@@ -253,19 +267,59 @@ int gemm_mmasp_launch(const uint32_t* meta, const uint32_t* values, const int8_t
     // fit in about 100 KB next to the slab, else fewer and more blocks along y
     const int tiles = (n + 7) / 8;
     const size_t slab = static_cast<size_t>(16 * a.rb) * (a.mpitch + a.vpitch) * 4;
-    int nt = tiles < kGqMaxTiles ? tiles : kGqMaxTiles;
+    GqShape s{};
+    s.nt = tiles < kGqMaxTiles ? tiles : kGqMaxTiles;
     auto xbytes = [&](int t) {
         const size_t act = static_cast<size_t>(8 * t) * a.xpitch, part = static_cast<size_t>(kGqWarps) * 16 * 8 * t * 4;
         return act > part ? act : part;
     };
-    while (nt > 1 && (nt == 3 || 2048 + kGqSignLutBytes + slab + xbytes(nt) > 110 * 1024)) --nt;
-    const size_t smem = 2048 + kGqSignLutBytes + slab + xbytes(nt);
-    if (smem > 200 * 1024) return fail(SPB_E_UNSUPPORTED, "%s: %d columns do not fit", name, cols);
-    void (*kernel)(GqArgs) = nt == 1 ? gemm_mmasp_kernel<1, false> : nt == 2 ? gemm_mmasp_kernel<2, false> : gemm_mmasp_kernel<4, false>;
-    if (a.ep.out) kernel = nt == 1 ? gemm_mmasp_kernel<1, true> : nt == 2 ? gemm_mmasp_kernel<2, true> : gemm_mmasp_kernel<4, true>;
-    if (int rc = ensure_dynamic_smem(name, kernel, smem)) return rc;
-    const dim3 grid((rows + 16 * a.rb - 1) / (16 * a.rb), (tiles + nt - 1) / nt);
-    return launch(name, kernel, grid, dim3(kGqThreads), smem, stream, a);
+    while (s.nt > 1 && (s.nt == 3 || 2048 + kGqSignLutBytes + slab + xbytes(s.nt) > 110 * 1024)) --s.nt;
+    s.smem = 2048 + kGqSignLutBytes + slab + xbytes(s.nt);
+    for (int i = 0; i < nmat; ++i) {
+        a.m[i] = GqMat{mats[i].meta, mats[i].values, mats[i].out, mats[i].gamma, mats[i].rows, mats[i].meta_stride, mats[i].values_stride, s.blocks_x};
+        s.blocks_x += (mats[i].rows + 16 * a.rb - 1) / (16 * a.rb);
+    }
+    s.blocks_y = (tiles + s.nt - 1) / s.nt;
+    return s;
+}
+
+// Whether this form is the faster one where it applies.  It starts sooner than the tcgen05 form (some 3 against 4 us for a
+// small product) and pays a pass of re-encoding per eight or sixteen batch rows (us, this form / tcgen05, half output where
+// not said):
+//   up to 8 batch rows while its blocks run at once, two per SM, or the matrix is small: 6912 x 6912, n = 2: 7.3 / 10.0;
+//     8192 x 6912, n = 8: 8.2 / 10.2;  2560 x 14336, n = 8 (a wave and a bit, one block per SM): 13.3 / 9.2;  28672 x 5632,
+//     n = 2: 20.3 / 16.0;  a half output's scales cost it more on short rows: 2560 x 512, n = 8: 3.7 / 3.6, 2560 x 256,
+//     n = 8, int32: 2.9 / 3.2;
+//   9 to 32 while no SM has a second block, a row block is shared by two warps or more and a block takes at most sixteen batch
+//     rows: 1001 x 6912, n = 16: 5.1 / 6.3;  256 x 5632, n = 32: 4.7 / 5.5;  14336 x 2048, n = 16: 10.0 / 6.7;  640 x 2560,
+//     n = 32: 8.8 / 5.4;  shorter rows for few of them or int32: 2048 x 2560, n = 9: 4.9 / 5.6;  6912 x 2560, n = 16: 7.2 / 6.7;
+//     2048 x 1024, n = 9, int32: 3.8 / 4.5, half 4.3 / 4.3.
+bool gemm_mmasp_preferred(const TcspMat* mats, int nmat, int cols, int n, bool half_out) {
+    if (n > 32) return false;
+    GqArgs a{};
+    const GqShape s = gq_shape(a, mats, nmat, cols, n);
+    const long long blocks = static_cast<long long>(s.blocks_x) * s.blocks_y;
+    long long rows = 0;
+    for (int i = 0; i < nmat; ++i) rows += mats[i].rows;
+    if (n > 8)
+        return cols >= (!half_out ? 1024 : rows <= 2048 ? 2048 : 4096) && a.ks >= 2 && s.nt <= 2 && blocks <= sm_count();
+    if (half_out && cols < 1024 && n > 4 && rows <= 8192) return false;
+    const int per_sm = s.smem > 112 * 1024 ? 1 : 2;
+    return blocks <= static_cast<long long>(per_sm) * sm_count() || (cols < 8192 && rows * cols <= 60ll * 1000 * 1000);
+}
+
+// absmax: row scales, the outputs are half; without, int32 sums
+int gemm_mmasp_launch(const TcspMat* mats, int nmat, const int8_t* X, const float* absmax, int cols, int n, void* stream) {
+    const char* name = "spb_sparse_ternary_gemm(mma.sp)";
+    GqArgs a{};
+    const GqShape s = gq_shape(a, mats, nmat, cols, n);
+    a.X = X;
+    a.absmax = absmax;
+    if (s.smem > 200 * 1024) return fail(SPB_E_UNSUPPORTED, "%s: %d columns do not fit", name, cols);
+    void (*kernel)(GqArgs) = s.nt == 1 ? gemm_mmasp_kernel<1, false> : s.nt == 2 ? gemm_mmasp_kernel<2, false> : gemm_mmasp_kernel<4, false>;
+    if (absmax) kernel = s.nt == 1 ? gemm_mmasp_kernel<1, true> : s.nt == 2 ? gemm_mmasp_kernel<2, true> : gemm_mmasp_kernel<4, true>;
+    if (int rc = ensure_dynamic_smem(name, kernel, s.smem)) return rc;
+    return launch(name, kernel, dim3(s.blocks_x, s.blocks_y), dim3(kGqThreads), s.smem, stream, a);
 }
 
 }  // namespace spb

@@ -20,6 +20,11 @@ struct TcspMat {
 // has; meta and values at their natural 4-byte alignment.
 int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const float* absmax, int cols, int n, void* stream);
 
+// gemm_mmasp.cu: the same on the warp-level sparse MMA; where it applies, and where it is the faster form
+bool gemm_mmasp_supported(const TcspMat* mats, int nmat, const int8_t* X, int cols, int n);
+bool gemm_mmasp_preferred(const TcspMat* mats, int nmat, int cols, int n, bool half_out);
+int gemm_mmasp_launch(const TcspMat* mats, int nmat, const int8_t* X, const float* absmax, int cols, int n, void* stream);
+
 // gemm.cu: BitLinear layers of one width on n quantised rows (scaled half outputs); acc_workspace: n * max rows int32, for the
 // forms that need it
 int bitlinear_gemm_group(const TcspMat* mats, int nmat, const int8_t* Xq, const float* absmax, int cols, int n,
