@@ -160,6 +160,12 @@ int spb_gemm_tc_timeouts(void);
  * the stream.  Returns SPB_E_TIMEOUT (the expected answer: the wait ran out and was reported) or SPB_E_CUDA.
  * Nothing is left in flight and the context stays usable. */
 int spb_debug_bounded_wait_selftest(long long limit_cycles, void* stream);
+/* Testing aid, no counterpart in the reference: the attention that spb_engine_prefill runs, T tokens (rows of num_heads *
+ * head_dim half in Q and out) at positions *d_pos .. *d_pos + T - 1 over caches of (num_kv_heads, max_seq_len, head_dim)
+ * half that hold them, with scale > 0.  SPB_E_UNSUPPORTED for shapes that the engine takes another way. */
+int spb_debug_prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads,
+                                int num_kv_heads, int head_dim, int max_seq_len, float scale, const int* d_pos,
+                                void* stream);
 
 /* ---- transformer kernels: include/spbitnet/inference_kernels.h ------------------- */
 

@@ -3,8 +3,10 @@
 //
 // A block takes the G query heads of one KV head and R tiles of 16 tokens, a warp one (head, tile): the 16 tokens are
 // the rows of mma.sync m16n8k16.  K and V go through shared memory in tiles of 64 positions, two in flight, read once
-// for all warps of the block.  Scores, running maximum, sum and output are fp32.  The exponentials enter the second
-// product as the sum of two halves (value and remainder, 22 bits), so nothing is rounded to half that was fp32 before.
+// for all warps of the block.  Scores, running maximum, sum and output are fp32.  A weight enters the second product as the sum
+// of two halves, value and remainder, of 2^15 times itself: the factor cancels against the sum of the weights, the largest
+// weight is still a half, and weights down to 2^-29 of the row's largest keep 22 bits (without it a weight below 2^-14 lost
+// bits and one below 2^-25 all of them, while the sum it is divided by still had it).
 // Tiles of positions start at multiples of 64 whatever the chunk, and a tile past a row's own position leaves the row
 // untouched, so a row's bits do not depend on how a prompt is cut into calls.
 //
@@ -22,6 +24,7 @@ namespace {
 
 constexpr int kPaTile = 64;  // positions per K / V tile
 constexpr int kPaRows = 16;  // tokens per warp
+constexpr float kPaFactor = 32768.0f;  // of the weights: the largest, this, is a half
 
 __device__ __forceinline__ void pa_ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -135,7 +138,6 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                     pa_mma(s[2 * nb], qf[k], b[0], b[1]);
                     pa_mma(s[2 * nb + 1], qf[k], b[2], b[3]);
                 }
-            float na = ma, nb_ = mb;
             if ((j + 1) * kPaTile - 1 > start + tok0) {  // some of the tile's positions are past some of the warp's rows
 #pragma unroll
                 for (int i = 0; i < kPaTile / 8; ++i) {
@@ -146,10 +148,9 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                     if (p + 1 > pb) s[i][3] = -INFINITY;
                 }
             }
+            float na = -INFINITY, nb_ = -INFINITY;
 #pragma unroll
             for (int i = 0; i < kPaTile / 8; ++i) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) s[i][c] *= scale_log2;
                 na = fmaxf(na, fmaxf(s[i][0], s[i][1]));
                 nb_ = fmaxf(nb_, fmaxf(s[i][2], s[i][3]));
             }
@@ -158,6 +159,8 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                 na = fmaxf(na, __shfl_xor_sync(0xFFFFFFFFu, na, off));
                 nb_ = fmaxf(nb_, __shfl_xor_sync(0xFFFFFFFFu, nb_, off));
             }
+            na = fmaxf(ma, na * scale_log2);  // scale > 0
+            nb_ = fmaxf(mb, nb_ * scale_log2);
             // position 0 is visible to every row, so the maxima are finite from the first tile on; past the first few tiles
             // they rarely move, and a factor of one is not multiplied
             if (__any_sync(0xFFFFFFFFu, !(na == ma && nb_ == mb))) {
@@ -180,10 +183,10 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float* e = s[2 * kk + h];
-                    e[0] = pa_exp2(e[0] - ma);
-                    e[1] = pa_exp2(e[1] - ma);
-                    e[2] = pa_exp2(e[2] - mb);
-                    e[3] = pa_exp2(e[3] - mb);
+                    e[0] = kPaFactor * pa_exp2(fmaf(e[0], scale_log2, -ma));
+                    e[1] = kPaFactor * pa_exp2(fmaf(e[1], scale_log2, -ma));
+                    e[2] = kPaFactor * pa_exp2(fmaf(e[2], scale_log2, -mb));
+                    e[3] = kPaFactor * pa_exp2(fmaf(e[3], scale_log2, -mb));
                     la += e[0] + e[1];
                     lb += e[2] + e[3];
                     pa_split(e[0], e[1], hi[2 * h], lo[2 * h]);
@@ -233,7 +236,7 @@ bool prefill_attention_supported(int num_heads, int num_kv_heads, int head_dim) 
 int prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads, int num_kv_heads,
                       int head_dim, int max_seq_len, float scale, const int* d_pos, void* stream) {
     const int G = num_heads / num_kv_heads;
-    const int R = max(1, 4 / G);  // at least four warps share a K / V tile
+    const int R = max(1, 4 / G);  // four warps or more share a K / V tile, three where G = 3
     const float scale_log2 = scale * 1.44269504088896340736f;
     const size_t smem = 4 * static_cast<size_t>(kPaTile) * head_dim * 2;
     auto kernel = head_dim == 64 ? prefill_attention_kernel<64> : prefill_attention_kernel<128>;
@@ -244,3 +247,15 @@ int prefill_attention(const void* Q, const void* K, const void* V, void* out, in
 }
 
 }  // namespace spb
+
+extern "C" int spb_debug_prefill_attention(const void* Q, const void* K, const void* V, void* out, int T, int num_heads,
+                                           int num_kv_heads, int head_dim, int max_seq_len, float scale, const int* d_pos,
+                                           void* stream) {
+    using namespace spb;
+    const char* name = "spb_debug_prefill_attention";
+    if (!Q || !K || !V || !out || !d_pos || T < 1 || max_seq_len < T || !(scale > 0.0f)) return fail(SPB_E_INVALID, "%s: bad arguments", name);
+    if (!prefill_attention_supported(num_heads, num_kv_heads, head_dim) ||
+        ((reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(out)) & 15u))
+        return fail(SPB_E_UNSUPPORTED, "%s: shape", name);
+    return prefill_attention(Q, K, V, out, T, num_heads, num_kv_heads, head_dim, max_seq_len, scale, d_pos, stream);
+}

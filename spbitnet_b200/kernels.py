@@ -66,6 +66,13 @@ def debug_grid_barrier_selftest(limit_cycles: int = 200000, stream=None) -> int:
     return load().spb_debug_grid_barrier_selftest(int(limit_cycles), _stream(stream))
 
 
+def debug_prefill_attention(Q, K, V, out, T, num_heads, num_kv_heads, head_dim, max_seq_len, scale, d_pos, stream=None):
+    """The prompt attention of InferenceEngine.prefill by itself (testing aid): Q and out (T, heads, head_dim) half, caches
+    (kv heads, max_seq_len, head_dim) half, d_pos the first token's position (int32, device)."""
+    check(load().spb_debug_prefill_attention(_p(Q), _p(K), _p(V), _p(out), T, num_heads, num_kv_heads, head_dim, max_seq_len,
+                                             float(scale), _p(d_pos), _stream(stream)))
+
+
 # ---- sparse_ternary_kernels.h ---------------------------------------------------------
 
 def sparse_ternary_unpack_gpu(meta, values, out, rows, cols, meta_row_stride, values_row_stride, stream=None):

@@ -1,0 +1,63 @@
+"""The prompt attention kernel's own output against float64: weights far below the row's largest, scores of both signs and
+sizes."""
+import numpy as np
+import pytest
+import torch
+
+from spbitnet_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(q, k, v, first, scale):
+    T, nh, hd = q.shape
+    nkv, max_seq, _ = k.shape
+    out = torch.full_like(q, 7.0)
+    K.debug_prefill_attention(q, k, v, out, T, nh, nkv, hd, max_seq, scale, torch.tensor([first], dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    return out
+
+
+def _exact(q, k, v, first, scale):
+    """Row by row over the positions the row sees, float64."""
+    T, nh, hd = q.shape
+    group = nh // k.shape[0]
+    out = torch.empty((T, nh, hd), dtype=torch.float64, device="cuda")
+    kd, vd = k.double().repeat_interleave(group, 0), v.double().repeat_interleave(group, 0)
+    for t in range(T):
+        n = first + t + 1
+        w = torch.softmax(torch.einsum("hd,hnd->hn", q[t].double(), kd[:, :n]) * scale, -1)
+        out[t] = torch.einsum("hn,hnd->hd", w, vd[:, :n])
+    return out
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("bits", [13, 20, 26, 28])
+def test_many_small_weights(head_dim, bits):
+    """One position with nearly all of the weight and a value of zero, thousands with a weight of 2^-bits of it: their sum is
+    the output.  Rounded to half (2^-11) it has to be right to 2^-11 + what 22 bits of each weight lose."""
+    n, T, nh, nkv = 4000, 20, 4, 2
+    scale = head_dim ** -0.5
+    q = torch.zeros((T, nh, head_dim), dtype=torch.float16, device="cuda")
+    k = torch.zeros((nkv, 4096, head_dim), dtype=torch.float16, device="cuda")
+    v = torch.ones_like(k)
+    q[..., 0] = 1.0
+    k[:, 0, 0] = bits * np.log(2.0) / scale
+    v[:, 0] = 0.0
+    got, want = _run(q, k, v, n, scale).double(), _exact(q, k, v, n, scale)
+    assert ((got - want).abs() <= 2.0 ** -10.9 * want + 2.0 ** -25).all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(3, 3, 64), (4, 1, 128), (8, 1, 64), (6, 2, 128)])
+@pytest.mark.parametrize("spread", [0.2, 1.0, 6.0])
+def test_random(heads, kv_heads, head_dim, spread):
+    """2^-11 of the value for its rounding to half; sums of up to 700 fp32 products and weights with a relative error of 2^-20
+    or so from the exponential of a score of up to 200 add 2^-18 of the largest value."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(heads)
+    first, T = 601, 99
+    q, k, v = ((s * torch.randn(shape, generator=g, device="cuda")).half()
+               for s, shape in [(spread, (T, heads, head_dim)), (1.0, (kv_heads, 768, head_dim)), (1.0, (kv_heads, 768, head_dim))])
+    scale = head_dim ** -0.5
+    got, want = _run(q, k, v, first, scale).double(), _exact(q, k, v, first, scale)
+    assert ((got - want).abs() <= 2.0 ** -10.9 * want.abs() + 2.0 ** -16).all()
