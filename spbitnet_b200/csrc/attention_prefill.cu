@@ -10,6 +10,11 @@
 // Tiles of positions start at multiples of 64 whatever the chunk, and a tile past a row's own position leaves the row
 // untouched, so a row's bits do not depend on how a prompt is cut into calls.
 //
+// Sums on the tensor core are cut off at each addition, not rounded.  Neither product therefore keeps one accumulator for long:
+// scores are formed in two chains of four or fewer, a tile of positions gives its part of the output in accumulators of its own,
+// which are added up in fp32.  (One accumulator over 4000 positions came out low by some 2^-16 and moved one rounding to half in
+// 33; so one in 700, a serial fp32 sum one in 370.  3 % of the time.)
+//
 // Bound: 20 heads of 128 over 1800 positions keep the tensor pipe busy for half of the active cycles and the chip active for
 // 70 % of them (245 blocks of unequal length on 148 SMs).  A block per (head, token) that walks the positions serially, used
 // before, re-read K and V once per head and token: 2176 us per chunk of 1024 or 776 tokens; this kernel 75 us, and 66 us since
@@ -125,19 +130,22 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
         if (tok0 < T && j * kPaTile <= start + min(tok0 + kPaRows, T) - 1) {  // else: every position is past the warp's rows
             float s[kPaTile / 8][4];
 #pragma unroll
-            for (int i = 0; i < kPaTile / 8; ++i)
+            for (int nb = 0; nb < kPaTile / 16; ++nb) {
+                float c0[2][4] = {}, c1[2][4] = {};
 #pragma unroll
-                for (int c = 0; c < 4; ++c) s[i][c] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < HD / 16; ++k)
-#pragma unroll
-                for (int nb = 0; nb < kPaTile / 16; ++nb) {
+                for (int k = 0; k < HD / 16; ++k) {
                     const int r = nb * 16 + (lane & 7) + ((lane >> 4) << 3), c = 2 * k + ((lane >> 3) & 1);
                     uint32_t b[4];
                     pa_ldsm4(b, kb + r * kRowBytes + ((c ^ (r & 7)) << 4));
-                    pa_mma(s[2 * nb], qf[k], b[0], b[1]);
-                    pa_mma(s[2 * nb + 1], qf[k], b[2], b[3]);
+                    pa_mma(c0[k & 1], qf[k], b[0], b[1]);
+                    pa_mma(c1[k & 1], qf[k], b[2], b[3]);
                 }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    s[2 * nb][c] = c0[0][c] + c0[1][c];
+                    s[2 * nb + 1][c] = c1[0][c] + c1[1][c];
+                }
+            }
             if ((j + 1) * kPaTile - 1 > start + tok0) {  // some of the tile's positions are past some of the warp's rows
 #pragma unroll
                 for (int i = 0; i < kPaTile / 8; ++i) {
@@ -177,9 +185,9 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                     o[i][3] *= cb;
                 }
             }
+            uint32_t hi[kPaTile / 16][4], lo[kPaTile / 16][4];
 #pragma unroll
-            for (int kk = 0; kk < kPaTile / 16; ++kk) {
-                uint32_t hi[4], lo[4];
+            for (int kk = 0; kk < kPaTile / 16; ++kk)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float* e = s[2 * kk + h];
@@ -189,18 +197,26 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
                     e[3] = kPaFactor * pa_exp2(fmaf(e[3], scale_log2, -mb));
                     la += e[0] + e[1];
                     lb += e[2] + e[3];
-                    pa_split(e[0], e[1], hi[2 * h], lo[2 * h]);
-                    pa_split(e[2], e[3], hi[2 * h + 1], lo[2 * h + 1]);
+                    pa_split(e[0], e[1], hi[kk][2 * h], lo[kk][2 * h]);
+                    pa_split(e[2], e[3], hi[kk][2 * h + 1], lo[kk][2 * h + 1]);
                 }
 #pragma unroll
-                for (int nb = 0; nb < HD / 16; ++nb) {
+            for (int nb = 0; nb < HD / 16; ++nb) {
+                float d0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int kk = 0; kk < kPaTile / 16; ++kk) {
                     const int r = kk * 16 + (lane & 15), c = 2 * nb + (lane >> 4);
                     uint32_t b[4];
                     pa_ldsm4_t(b, vb + r * kRowBytes + ((c ^ (r & 7)) << 4));
-                    pa_mma(o[2 * nb], hi, b[0], b[1]);
-                    pa_mma(o[2 * nb + 1], hi, b[2], b[3]);
-                    pa_mma(o[2 * nb], lo, b[0], b[1]);
-                    pa_mma(o[2 * nb + 1], lo, b[2], b[3]);
+                    pa_mma(d0, lo[kk], b[0], b[1]);
+                    pa_mma(d1, lo[kk], b[2], b[3]);
+                    pa_mma(d0, hi[kk], b[0], b[1]);
+                    pa_mma(d1, hi[kk], b[2], b[3]);
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    o[2 * nb][c] += d0[c];
+                    o[2 * nb + 1][c] += d1[c];
                 }
             }
         }

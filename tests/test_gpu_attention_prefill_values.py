@@ -61,3 +61,18 @@ def test_random(heads, kv_heads, head_dim, spread):
     scale = head_dim ** -0.5
     got, want = _run(q, k, v, first, scale).double(), _exact(q, k, v, first, scale)
     assert ((got - want).abs() <= 2.0 ** -10.9 * want.abs() + 2.0 ** -16).all()
+
+
+def test_long_sequence_without_bias():
+    """Equal weights over thousands of positive values: sums that a tensor core accumulates over the whole sequence come out low by
+    a few 2^-16 (each addition is cut off, not rounded), enough to move one rounding to half in thirty.  Rounded once, an fp32
+    result moves one in a few hundred."""
+    heads, kv_heads, head_dim, T, first = 4, 2, 128, 32, 4000
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    q = 0.1 * torch.randn((T, heads, head_dim), generator=g, device="cuda").half()
+    k = torch.randn((kv_heads, 4096, head_dim), generator=g, device="cuda").half()
+    v = 1.0 + torch.rand((kv_heads, 4096, head_dim), generator=g, device="cuda").half()
+    scale = head_dim ** -0.5
+    got, want = _run(q, k, v, first, scale), _exact(q, k, v, first, scale)
+    assert (got != want.half()).double().mean() < 0.01
