@@ -30,7 +30,12 @@
 //   of 128 has tight sign rows of 8 (mod 16) bytes, which no tensor map takes.  Warp 18 brings the signs by 8-byte asynchronous
 //   copies, four lanes per row and chunk, on the barrier that the bitmaps' copy completes.  28672 x 5504, n = 200: 27 us, in the
 //   form for any layout 217;  6912 x 3200, n = 64: 9.1 and 17.5;  5000 x 1408, n = 200: 7.5 and 17.1.
+// LAYOUT = kEdge: kTiled for widths that are no multiple of 128.
 // LAYOUT = kAny: any other: the re-encoding warps load their words themselves, eight warps copy the activation tiles.
+//
+// kEdge and kAny decode every bitmap as the reference's table has it, also those without two bits set: these layouts have
+// always been decoded by the table (6912 x 3204, n = 16, half: 12.2 -> 12.7 us).  The others take packed rows as the packing
+// rules make them.
 //
 // Every wait is bounded; a role whose wait runs out records it and leaves its loop, the others then run out of their own
 // bounds, the copy warps wait (bounded) for their copies in flight, tensor memory is freed and the block returns.
@@ -55,7 +60,7 @@ constexpr int kWsThreadsAny = 32 * (kWsXWarp + kWsCopyWarps);
 constexpr int kWsBarBytes = 512, kWsScaleBytes = 1024;
 constexpr int kWsSmemCap = 226 * 1024;
 
-enum WsLayout { kTiled = 0, kAny = 1, kSigns8 = 2 };
+enum WsLayout { kTiled = 0, kAny = 1, kSigns8 = 2, kEdge = 3 };
 
 struct WsMat {
     const uint32_t* meta;
@@ -116,6 +121,12 @@ __device__ __forceinline__ uint32_t ws_index_pairs(uint32_t m) {
     const uint32_t t2 = (0x22222222u & (~ml & ~m)) | (~0x22222222u & (m | ml));
     return (t1 & 0x55555555u) | (t2 & 0xAAAAAAAAu);
 }
+// Bit 4 g set: bitmap g has not two bits set.
+__device__ __forceinline__ uint32_t ws_odd_bitmaps(uint32_t m) {
+    m -= (m >> 1) & 0x55555555u;
+    const uint32_t x = ((m & 0x33333333u) + ((m >> 2) & 0x33333333u)) ^ 0x22222222u;  // counts of bits, 0 where two
+    return (x | (x >> 1) | (x >> 2)) & 0x11111111u;
+}
 // 32 sign bits -> 32 bytes of +1 / -1 in order.  Transposing the 4 x 4 bits of each 16-bit half puts the signs 4 r .. 4 r
 // + 3 at bit r of the half's four nibbles; a byte permute with the nibbles as selectors and a source whose byte i is -1
 // where bit r of i is set then yields those four bytes.  A selector's top bit means "replicate the sign", so the nibbles
@@ -140,7 +151,7 @@ __device__ __forceinline__ void ws_sign_bytes(uint32_t v, uint32_t (&w)[8]) {
 template <bool HALF_OUT, int LAYOUT, bool ROWS4>
 __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsAny, 1)
     gemm_tcsp_ws_kernel(const WsArgs a, const __grid_constant__ WsMaps maps) {
-    constexpr bool kMapped = LAYOUT != kAny, kAsyncSigns = LAYOUT == kSigns8;
+    constexpr bool kMapped = LAYOUT != kAny, kAsyncSigns = LAYOUT == kSigns8, kAnyBitmap = LAYOUT == kAny || LAYOUT == kEdge;
     extern __shared__ uint8_t ws_raw[];
     // [barriers][row scales] ... 1024-aligned: [A ring][activation ring][packed-word ring]; the epilogue's sums take the
     // place of the rings when the products are done
@@ -396,6 +407,18 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
                 vv = vn;
                 load_words(i + stride, mn, vn);
             }
+            uint32_t odd0 = 0, odd1 = 0, odd2 = 0, odd3 = 0;  // groups of the row whose bitmap has not two bits set
+            if (kAnyBitmap) {
+                const int left = row0 + wr < m.rows ? (a.cols >> 2) - 32 * (2 * (s0 + i) + thalf) : 0;  // the row's groups from here on
+                auto odd = [&](uint32_t word, int q) {
+                    const int g = left - 8 * q;
+                    return g <= 0 ? 0u : ws_odd_bitmaps(word) & (g >= 8 ? 0xFFFFFFFFu : (1u << (4 * g)) - 1u);
+                };
+                odd0 = odd(mm.x, 0);
+                odd1 = odd(mm.y, 1);
+                odd2 = odd(mm.z, 2);
+                odd3 = odd(mm.w, 3);
+            }
             if (row_tail || (s0 + i + 1) * kWsStepK > a.cols) {
                 mm.x = ws_fill_empty(mm.x);
                 mm.y = ws_fill_empty(mm.y);
@@ -403,8 +426,15 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
                 mm.w = ws_fill_empty(mm.w);
             }
             uint32_t w0[8], w1[8];
-            const uint32_t e0 = ws_index_pairs(mm.x), e1 = ws_index_pairs(mm.y), e2 = ws_index_pairs(mm.z),
-                           e3 = ws_index_pairs(mm.w);
+            uint32_t e0 = ws_index_pairs(mm.x), e1 = ws_index_pairs(mm.y), e2 = ws_index_pairs(mm.z), e3 = ws_index_pairs(mm.w);
+            // The table puts both signs of such a group on its first column: index pair {0, 1} with the bytes {s0 + s1, 0}, the bytes
+            // mended below.  (At an edge, groups past it were filled with {0, 1} above; an empty group inside gets the same.)
+            if (kAnyBitmap) {
+                e0 = (e0 & ~(odd0 * 15u)) | (odd0 << 2);
+                e1 = (e1 & ~(odd1 * 15u)) | (odd1 << 2);
+                e2 = (e2 & ~(odd2 * 15u)) | (odd2 << 2);
+                e3 = (e3 & ~(odd3 * 15u)) | (odd3 << 2);
+            }
             ws_sign_bytes(vv.x, w0);
             ws_sign_bytes(vv.y, w1);
             const int sA = ca.s;
@@ -422,6 +452,18 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sm + ws_swz(trow, thalf * 4 + c)), "r"(w[0]),
                              "r"(w[1]), "r"(w[2]), "r"(w[3])
                              : "memory");
+            }
+            if (kAnyBitmap && (odd0 | odd1 | odd2 | odd3)) {
+#pragma unroll 1
+                for (int g = 0; g < 32; ++g) {
+                    const uint32_t word = g < 8 ? odd0 : g < 16 ? odd1 : g < 24 ? odd2 : odd3;
+                    if (!((word >> (4 * (g & 7))) & 1u)) continue;
+                    const uint32_t signs = ((g < 16 ? vv.x : vv.y) >> (2 * (g & 15))) & 3u;
+                    const uint32_t pair = signs == 0 ? 2u : signs == 3 ? 0xFEu : 0u;  // s0 + s1 | 0 << 8
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(sm + ws_swz(trow, thalf * 4 + (g >> 3)) + 2 * (g & 7)),
+                                 "h"(static_cast<unsigned short>(pair))
+                                 : "memory");
+                }
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
@@ -786,17 +828,19 @@ int gemm_tcsp_ws_launch(const TcspMat* mats, int nmat, const int8_t* X, const fl
     a.timeouts = timeout_counter();
     a.wait_cycles = kWsWaitCycles;
     using Kernel = void (*)(WsArgs, WsMaps);
-    static const Kernel kernels[3][2][2] = {  // layout, half output, four rows on a boundary
+    static const Kernel kernels[4][2][2] = {  // layout, half output, four rows on a boundary
         {{gemm_tcsp_ws_kernel<false, kTiled, false>, gemm_tcsp_ws_kernel<false, kTiled, true>},
          {gemm_tcsp_ws_kernel<true, kTiled, false>, gemm_tcsp_ws_kernel<true, kTiled, true>}},
         {{gemm_tcsp_ws_kernel<false, kAny, false>, gemm_tcsp_ws_kernel<false, kAny, true>},
          {gemm_tcsp_ws_kernel<true, kAny, false>, gemm_tcsp_ws_kernel<true, kAny, true>}},
         {{gemm_tcsp_ws_kernel<false, kSigns8, false>, gemm_tcsp_ws_kernel<false, kSigns8, true>},
-         {gemm_tcsp_ws_kernel<true, kSigns8, false>, gemm_tcsp_ws_kernel<true, kSigns8, true>}}};
+         {gemm_tcsp_ws_kernel<true, kSigns8, false>, gemm_tcsp_ws_kernel<true, kSigns8, true>}},
+        {{gemm_tcsp_ws_kernel<false, kEdge, false>, gemm_tcsp_ws_kernel<false, kEdge, true>},
+         {gemm_tcsp_ws_kernel<true, kEdge, false>, gemm_tcsp_ws_kernel<true, kEdge, true>}}};
     bool rows4 = true;
     for (int i = 0; i < nmat; ++i)
         rows4 = rows4 && mats[i].rows % 4 == 0 && (reinterpret_cast<uintptr_t>(mats[i].out) & (absmax ? 7u : 15u)) == 0;
-    const Kernel kernel = kernels[!tiled ? kAny : signs16 ? kTiled : kSigns8][absmax != nullptr][rows4];
+    const Kernel kernel = kernels[!tiled ? kAny : cols % 128 ? kEdge : signs16 ? kTiled : kSigns8][absmax != nullptr][rows4];
     if (int rc = ensure_dynamic_smem(name, kernel, c.smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, (n + c.nt - 1) / c.nt, c.split);

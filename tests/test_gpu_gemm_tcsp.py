@@ -79,3 +79,33 @@ def test_sign_rows_on_eight_byte_boundaries(rows, cols, n, halves):
             assert (out.read(np.float16).reshape(n, rows).view(np.uint16) == wh.view(np.uint16)).all(), (stride, shift)
     finally:
         K.set_gemm_row_halves(old)
+
+
+@pytest.mark.parametrize("rows,cols,n,pad", [(40, 68, 5, 0), (300, 132, 40, 0), (130, 272, 17, 2), (150, 640, 21, 1), (257, 1036, 33, 0)])
+def test_bitmaps_without_two_bits_decode_as_the_table_has_them(rows, cols, n, pad):
+    """Layouts outside whole 128-column rows: any bitmap, both signs on the first column where it has not two bits set."""
+    rng = np.random.default_rng(rows)
+    ms, vs = (cols // 4 + 7) // 8 + pad, (cols // 4 + 15) // 16 + pad
+    if pad == 2:
+        ms, vs = (ms + 3) // 4 * 4, (vs + 3) // 4 * 4  # tensor maps take these rows
+    case = synth.gemm_case(rows, cols, n, seed=7)
+    meta = np.zeros((rows, ms), np.uint32)
+    values = rng.integers(0, 2**32, (rows, vs), dtype=np.uint64).astype(np.uint32)
+    meta[:, :case["meta"].reshape(rows, -1).shape[1]] = case["meta"].reshape(rows, -1)
+    for r in range(0, rows, 3):  # every third row: any bits in the row's own groups
+        for g in range(cols // 4):
+            meta[r, g // 8] = (int(meta[r, g // 8]) & ~(15 << (4 * (g % 8)))) | (int(rng.integers(0, 16)) << (4 * (g % 8)))
+    x = rng.integers(-127, 128, (n, cols)).astype(np.int8)
+    w = np.zeros((rows, cols), np.int64)
+    g = np.arange(cols // 4)
+    b = (meta[:, g // 8] >> (4 * (g % 8)).astype(np.uint32)) & 15
+    s = (values[:, g // 16] >> (2 * (g % 16)).astype(np.uint32)) & 3
+    for r in range(rows):
+        for k in g:
+            pos = [i for i in range(4) if (int(b[r, k]) >> i) & 1]
+            p0, p1 = pos if len(pos) == 2 else (0, 0)
+            w[r, 4 * k + p0] += -1 if s[r, k] & 1 else 1
+            w[r, 4 * k + p1] += -1 if s[r, k] & 2 else 1
+    Y = Guarded(n * rows * 4)
+    K.sparse_ternary_gemm_gpu(dev(meta), dev(values), dev(x), Y.ptr, rows, cols, n, ms, vs)
+    assert (Y.read(np.int32).reshape(n, rows) == x.astype(np.int64) @ w.T).all()
