@@ -166,15 +166,53 @@ def load() -> C.CDLL:
     return lib
 
 
+class CtypesCalls:
+    """The calls of csrc/py_calls.cpp through ctypes, some 5 us slower each: for an installation that was built without Python's
+    headers or is run by another Python than the one it was built for."""
+
+    def __init__(self, lib):
+        self._lib = lib
+
+    def __getattr__(self, name):
+        fn, kinds = getattr(self._lib, name), SIGNATURES[name][1]
+
+        def call(*args):
+            if len(args) != len(kinds):
+                raise TypeError(f"{len(kinds)} arguments wanted, {len(args)} given")
+            values = [_address(a) if kind is _p else float(a) if kind is _f else a for kind, a in zip(kinds[:-1], args)]
+            check(fn(*values, _stream_address(args[-1])))
+
+        setattr(self, name, call)
+        return call
+
+
+def _address(a):
+    return a if a is None or isinstance(a, int) else a.data_ptr()
+
+
+def _stream_address(stream):
+    if stream is None:
+        import torch
+        return torch.cuda.current_stream().cuda_stream
+    return stream if isinstance(stream, int) else stream.cuda_stream
+
+
+_calls = None
+
+
 def calls():
-    """The CPython module that calls the kernel entry points (csrc/py_calls.cpp), bound to the loaded library."""
-    lib = load()
-    try:
-        from . import _calls
-    except ImportError as e:
-        raise ImportError("spbitnet_b200/_calls is missing. Build it with `python -m spbitnet_b200.build`.") from e
-    _calls.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES},
-                check)
+    """What calls the kernel entry points of the loaded library: the CPython module built from csrc/py_calls.cpp, or ctypes
+    where there is none for this Python."""
+    global _calls
+    if _calls is None:
+        lib = load()
+        try:
+            from . import _calls as module
+        except ImportError:
+            _calls = CtypesCalls(lib)
+        else:
+            module.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES}, check)
+            _calls = module
     return _calls
 
 

@@ -38,11 +38,15 @@ def sources() -> list[Path]:
 
 
 def needs_build() -> bool:
-    if not LIB.exists() or not CALLS.exists():
+    if not LIB.exists() or (not CALLS.exists() and _python_headers()):
         return True
     t = LIB.stat().st_mtime
     deps = [p for p in CSRC.glob("*") if p.is_file()] + [HERE.parent / "include" / "spbitnet_b200.h"]
     return any(p.stat().st_mtime > t for p in deps)
+
+
+def _python_headers() -> bool:
+    return (Path(sysconfig.get_paths()["include"]) / "Python.h").exists()
 
 
 def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool) -> str:
@@ -77,9 +81,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     res = subprocess.run([nvcc, *LINK_FLAGS, "-o", str(LIB), *objs], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
-    # the CPython module that calls the entry points (bound to the loaded library at import, not linked)
+    # the CPython module that calls the entry points (bound to the loaded library at the first call, not linked); without
+    # Python's headers the package makes them through ctypes
     calls_src = CSRC / "py_calls.cpp"
-    if force or not CALLS.exists() or CALLS.stat().st_mtime < max(calls_src.stat().st_mtime, newest_header):
+    if not _python_headers():
+        print(f"{CALLS.name} not built: no Python.h in {sysconfig.get_paths()['include']}", file=sys.stderr)
+    elif force or not CALLS.exists() or CALLS.stat().st_mtime < max(calls_src.stat().st_mtime, newest_header):
         res = subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-I",
                               sysconfig.get_paths()["include"], "-o", str(CALLS), str(calls_src)], capture_output=True, text=True)
         if res.returncode != 0:

@@ -34,7 +34,7 @@ enum Index {
 };
 void* g_fn[kCount];
 PyObject *g_data_ptr, *g_cuda_stream;                      // attribute names
-PyObject *g_get_device, *g_get_raw_stream, *g_current_stream;  // torch._C._cuda_getDevice, _cuda_getCurrentRawStream; torch.cuda.current_stream
+PyObject *g_get_device = nullptr, *g_get_raw_stream = nullptr;  // torch._C._cuda_getDevice, _cuda_getCurrentRawStream
 PyObject* g_check = nullptr;  // called with a status other than 0
 bool g_cuda_ready = false;
 
@@ -55,16 +55,35 @@ bool to_pointer(PyObject* o, void** out) {
     return !PyErr_Occurred();
 }
 
+PyObject* attribute(const char* module, const char* name) {
+    PyObject* m = PyImport_ImportModule(module);
+    if (!m) return nullptr;
+    PyObject* a = PyObject_GetAttrString(m, name);
+    Py_DECREF(m);
+    return a;
+}
+
+// At the first call that leaves the stream to torch: also initialises CUDA there, as the first use of a stream does.
+bool init_torch_streams() {
+    if (!g_get_device) g_get_device = attribute("torch._C", "_cuda_getDevice");
+    if (!g_get_device) return false;
+    if (!g_get_raw_stream) g_get_raw_stream = attribute("torch._C", "_cuda_getCurrentRawStream");
+    if (!g_get_raw_stream) return false;
+    PyObject* current = attribute("torch.cuda", "current_stream");
+    if (!current) return false;
+    PyObject* s = PyObject_CallNoArgs(current);
+    Py_DECREF(current);
+    if (!s) return false;
+    Py_DECREF(s);
+    g_cuda_ready = true;
+    return true;
+}
+
 // None: torch's current stream of the current device; an address; or a stream object
 bool to_stream(PyObject* o, void** out) {
     PyObject* r = nullptr;
     if (o == Py_None) {
-        if (!g_cuda_ready) {  // initialises CUDA in torch, as the first use of a stream does
-            PyObject* s = PyObject_CallNoArgs(g_current_stream);
-            if (!s) return false;
-            Py_DECREF(s);
-            g_cuda_ready = true;
-        }
+        if (!g_cuda_ready && !init_torch_streams()) return false;
         PyObject* dev = PyObject_CallNoArgs(g_get_device);
         if (!dev) return false;
         r = PyObject_CallOneArg(g_get_raw_stream, dev);
@@ -157,22 +176,11 @@ PyMethodDef g_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_calls", "Kernel entry points of libspbitnet_b200.so", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
-PyObject* attribute(const char* module, const char* name) {
-    PyObject* m = PyImport_ImportModule(module);
-    if (!m) return nullptr;
-    PyObject* a = PyObject_GetAttrString(m, name);
-    Py_DECREF(m);
-    return a;
-}
-
 }  // namespace
 
 PyMODINIT_FUNC PyInit__calls() {
     g_data_ptr = PyUnicode_InternFromString("data_ptr");
     g_cuda_stream = PyUnicode_InternFromString("cuda_stream");
-    g_get_device = attribute("torch._C", "_cuda_getDevice");
-    g_get_raw_stream = attribute("torch._C", "_cuda_getCurrentRawStream");
-    g_current_stream = attribute("torch.cuda", "current_stream");
-    if (!g_data_ptr || !g_cuda_stream || !g_get_device || !g_get_raw_stream || !g_current_stream) return nullptr;
+    if (!g_data_ptr || !g_cuda_stream) return nullptr;
     return PyModule_Create(&g_module);
 }

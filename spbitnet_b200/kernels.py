@@ -12,7 +12,18 @@ import torch
 from . import _lib
 from ._lib import check, load
 
-_c = _lib.calls()  # converts tensors, addresses, None and streams; a status other than 0 raises SpbError
+
+class _Calls:
+    """The kernel entry points: tensors, addresses, None and streams in, SpbError for a status other than 0.  Looked up at the
+    first call of each: this module can be imported before the library is built."""
+
+    def __getattr__(self, name):
+        fn = getattr(_lib.calls(), name)
+        setattr(self, name, fn)
+        return fn
+
+
+_c = _Calls()
 
 
 def _p(t):
