@@ -814,13 +814,22 @@ extern "C" int spb_engine_seq_len(const spb_engine* e) { return e ? e->seq_len :
 extern "C" int spb_engine_copy_logits(spb_engine* e, float* h_logits) {
     if (!e || !h_logits) return fail(SPB_E_INVALID, "spb_engine_copy_logits: null pointer");
     SPB_ON_ENGINE_DEVICE(e);
-    // By way of pinned memory: a copy of 513 KB into fresh pageable memory (a caller that keeps every token's logits) took
-    // 260 us, page by page in the driver; this and the move into the fresh pages take 205 us.
+    // Into pageable memory by way of pinned memory: a copy of 513 KB into fresh pages (a caller that keeps every token's logits)
+    // took 260 us, page by page in the driver; this and the move into the fresh pages take 205 us.  What the runtime knows
+    // (pinned memory, or an address that no host code may touch) is its own to copy to.
     const size_t bytes = sizeof(float) * static_cast<size_t>(e->cfg.vocab_size);
-    std::lock_guard<std::mutex> one(e->h_logits_use);
-    SPB_CUDA(cudaMemcpyAsync(e->h_logits ? e->h_logits : h_logits, e->logits, bytes, cudaMemcpyDeviceToHost, e->stream));
-    SPB_CUDA(cudaStreamSynchronize(e->stream));
-    if (e->h_logits) std::memcpy(h_logits, e->h_logits, bytes);
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, h_logits) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (pageable && e->h_logits) {
+        std::lock_guard<std::mutex> one(e->h_logits_use);
+        SPB_CUDA(cudaMemcpyAsync(e->h_logits, e->logits, bytes, cudaMemcpyDeviceToHost, e->stream));
+        SPB_CUDA(cudaStreamSynchronize(e->stream));
+        std::memcpy(h_logits, e->h_logits, bytes);
+    } else {
+        SPB_CUDA(cudaMemcpyAsync(h_logits, e->logits, bytes, cudaMemcpyDeviceToHost, e->stream));
+        SPB_CUDA(cudaStreamSynchronize(e->stream));
+    }
     return check_timeouts(e, "spb_engine_copy_logits");
 }
 
