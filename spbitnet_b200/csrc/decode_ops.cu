@@ -276,7 +276,7 @@ constexpr int kOutLoads = 4;
 __global__ void __launch_bounds__(kBlock) attention_output_cluster_kernel(
     const float* __restrict__ scores, const __half* __restrict__ V, __half* __restrict__ out, int num_heads, int num_kv_heads,
     int head_dim, int max_seq_len, int seq_len) {
-    __shared__ float part[kBlock * 8];  // npg x head_dim
+    __shared__ __align__(16) float part[kBlock * 8];  // npg x head_dim, written four at a time
     __shared__ float sum[kBlock * 8];   // head_dim
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
