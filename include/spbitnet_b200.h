@@ -379,6 +379,9 @@ int spb_engine_decode_is_persistent(const spb_engine* e);
 /* Test aid: two blocks at a grid barrier that expects three; both waits run out after limit_cycles (clamped),
  * the run-out is counted, the kernel returns.  Returns SPB_E_TIMEOUT when that happened as it must. */
 int spb_debug_grid_barrier_selftest(long long limit_cycles, void* stream);
+/* Testing aid, no counterpart in the reference: the elements other than zero of an engine's K (values = 0) or V (1)
+ * caches, all layers and all positions, counted on the host; negative: a status. */
+long long spb_debug_engine_cache_nonzeros(spb_engine* e, int values);
 /* Diagnostic: persistent decode kernels enqueued (or captured) after this call record stage times.  d_trace is device
  * memory for 2 x 4096 64-bit words, or NULL to switch the recording off: thread 0 of the first block writes words
  * [0, 4096), thread 0 of the last block [4096, 8192); word 20 * layer + k is the global nanosecond timer at point k of
@@ -476,6 +479,8 @@ int spb_shard_engine_seq_len(const spb_shard_engine* e);
 int spb_shard_engine_step(spb_shard_engine* e, const int* tokens);
 /* h_logits_rows: batch x (stop - start of which = 7) floats (HOST): this rank's vocabulary rows of the last step. */
 int spb_shard_engine_copy_logits(spb_shard_engine* e, float* h_logits_rows);
+/* Testing aid: spb_debug_engine_cache_nonzeros of this engine. */
+long long spb_debug_shard_engine_cache_nonzeros(spb_shard_engine* e, int values);
 /* The greedy loop of src/main.cpp:266-300 for `batch` sequences: prompt is n_prompt x batch token ids (HOST,
  * position-major), out_tokens max_tokens x batch.  Feeds prompt[0 .. n_prompt-2], then generates max_tokens tokens
  * from prompt[n_prompt-1]; no EOS stop.  Returns max_tokens or a negative status. */

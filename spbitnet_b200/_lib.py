@@ -72,6 +72,8 @@ SIGNATURES = {
     "spb_debug_bounded_wait_selftest": (_i, [C.c_longlong, _p]),
     "spb_debug_grid_barrier_selftest": (_i, [C.c_longlong, _p]),
     "spb_debug_prefill_attention": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _p, _p]),
+    "spb_debug_engine_cache_nonzeros": (C.c_longlong, [_p, _i]),
+    "spb_debug_shard_engine_cache_nonzeros": (C.c_longlong, [_p, _i]),
     "spb_debug_set_decode_trace": (None, [_p]),
     "spb_rms_norm": (_i, [_p, _p, _p, _i, _f, _p]),
     "spb_absmax_quantize": (_i, [_p, _p, _p, _i, _p]),

@@ -88,6 +88,18 @@ cudaError_t clear_cache_positions(void* cache, int layers, size_t layer_bytes, s
     return cudaSuccess;
 }
 
+long long count_nonzero_halves(const void* p, size_t bytes, cudaStream_t stream) {
+    std::vector<uint16_t> host(bytes / 2);
+    if (cudaMemcpyAsync(host.data(), p, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SPB_E_CUDA, "reading device memory failed");
+    }
+    long long n = 0;
+    for (const uint16_t h : host) n += h != 0;
+    return n;
+}
+
 }  // namespace spb
 
 extern "C" int spb_gemm_tc_timeouts(void) {

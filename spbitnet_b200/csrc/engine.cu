@@ -784,6 +784,12 @@ extern "C" int spb_engine_reset(spb_engine* e) {
     return SPB_OK;
 }
 
+extern "C" long long spb_debug_engine_cache_nonzeros(spb_engine* e, int values) {
+    if (!e) return fail(SPB_E_INVALID, "spb_debug_engine_cache_nonzeros: null handle");
+    SPB_ON_ENGINE_DEVICE(e);
+    return count_nonzero_halves(values ? e->vcache : e->kcache, e->kv_bytes_per_layer * e->cfg.num_hidden_layers, e->stream);
+}
+
 extern "C" int spb_engine_set_decode_mode(spb_engine* e, int mode) {
     if (!e) return fail(SPB_E_INVALID, "spb_engine_set_decode_mode: null handle");
     if (mode < 0 || mode > 4) return fail(SPB_E_INVALID, "spb_engine_set_decode_mode: mode %d", mode);

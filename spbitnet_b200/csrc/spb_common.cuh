@@ -98,6 +98,8 @@ int launch_clustered(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3
 // apart, on `stream` (core.cu).
 cudaError_t clear_cache_positions(void* cache, int layers, size_t layer_bytes, size_t rows, int max_positions, size_t row_bytes,
                                   int positions, cudaStream_t stream);
+// 16-bit words other than zero among `bytes` of device memory, read through the host; negative on failure (core.cu)
+long long count_nonzero_halves(const void* p, size_t bytes, cudaStream_t stream);
 
 // griddepcontrol.launch_dependents: lets the next grid on the stream begin its independent prologue
 // (weight prefetch).  Harmless without PDL.  Most kernels call it first thing; the tensor-core GEMV
