@@ -8,7 +8,8 @@
 // weight is still a half, and weights down to 2^-29 of the row's largest keep 22 bits (without it a weight below 2^-14 lost
 // bits and one below 2^-25 all of them, while the sum it is divided by still had it).
 // Tiles of positions start at multiples of 64 whatever the chunk, and a tile past a row's own position leaves the row
-// untouched, so a row's bits do not depend on how a prompt is cut into calls.
+// untouched, so a row's bits do not depend on how a prompt is cut into calls (while V is finite: a block that comes upon other
+// values forms its rows again, pa_rows_one_by_one, whose sums are in another order).
 //
 // Sums on the tensor core are cut off at each addition, not rounded.  Neither product therefore keeps one accumulator for long:
 // scores are formed in two chains of four or fewer, a tile of positions gives its part of the output in accumulators of its own,
@@ -59,6 +60,50 @@ __device__ __forceinline__ void pa_split(float a, float b, uint32_t& hi, uint32_
     const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// A warp's 16 rows position by position, for a block whose outputs are not all finite: an infinity or a NaN of V is to reach the
+// rows that see its position, but in a product on the tensor core a weight of zero makes NaN of it, and so do the two halves of
+// a weight.  Out of line and not tuned: as a second turn of the kernel's own loop it made that loop 9 % slower.
+template <int HD>
+__device__ __noinline__ void pa_rows_one_by_one(const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
+                                                __half* __restrict__ out, int tok0, int T, int start, int num_heads, int head, float scale_log2) {
+    constexpr int kDims = HD / 32;
+    const int lane = threadIdx.x & 31;
+    for (int t = tok0; t < min(tok0 + kPaRows, T); ++t) {
+        const __half* q = Q + (static_cast<size_t>(t) * num_heads + head) * HD;
+        const int n = start + t + 1;
+        float m = -INFINITY, l = 0.0f, o[kDims];
+#pragma unroll
+        for (int i = 0; i < kDims; ++i) o[i] = 0.0f;
+        for (int p0 = 0; p0 < n; p0 += 32) {
+            const int p = p0 + lane;
+            float s = -INFINITY;
+            if (p < n) {
+                s = 0.0f;
+                for (int d = 0; d < HD; ++d) s = fmaf(__half2float(q[d]), __half2float(K[static_cast<size_t>(p) * HD + d]), s);
+                s *= scale_log2;
+            }
+            float mn = s;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, off));
+            mn = fmaxf(m, mn);
+            const float corr = exp2f(m - mn), e = p < n ? exp2f(s - mn) : 0.0f;
+            m = mn;
+            l = l * corr + e;
+#pragma unroll
+            for (int i = 0; i < kDims; ++i) o[i] *= corr;
+            for (int r = 0; r < min(32, n - p0); ++r) {
+                const float w = __shfl_sync(0xFFFFFFFFu, e, r);
+#pragma unroll
+                for (int i = 0; i < kDims; ++i) o[i] = fmaf(w, __half2float(V[static_cast<size_t>(p0 + r) * HD + 32 * i + lane]), o[i]);
+            }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, off);
+#pragma unroll
+        for (int i = 0; i < kDims; ++i) out[(static_cast<size_t>(t) * num_heads + head) * HD + 32 * i + lane] = __float2half_rn(o[i] / l);
+    }
 }
 
 template <int HD>
@@ -226,6 +271,15 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(
     for (int off = 1; off < 4; off <<= 1) {
         la += __shfl_xor_sync(0xFFFFFFFFu, la, off);
         lb += __shfl_xor_sync(0xFFFFFFFFu, lb, off);
+    }
+    float z = 0.0f;  // 0 times anything finite
+#pragma unroll
+    for (int i = 0; i < HD / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) z = fmaf(o[i][c], 0.0f, z);
+    if (__syncthreads_or(z != 0.0f)) {
+        pa_rows_one_by_one<HD>(Q, reinterpret_cast<const __half*>(kg), reinterpret_cast<const __half*>(vg), out, tok0, T, start, num_heads, head, scale_log2);
+        return;
     }
     const float ia = 1.0f / la, ib = 1.0f / lb;
     const int ra = tok0 + g, rb = tok0 + g + 8;

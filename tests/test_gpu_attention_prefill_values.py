@@ -1,5 +1,5 @@
 """The prompt attention kernel's own output against float64: weights far below the row's largest, scores of both signs and
-sizes."""
+sizes, and values that are not finite, at positions a row sees and at ones it does not."""
 import numpy as np
 import pytest
 import torch
@@ -76,3 +76,44 @@ def test_long_sequence_without_bias():
     scale = head_dim ** -0.5
     got, want = _run(q, k, v, first, scale), _exact(q, k, v, first, scale)
     assert (got != want.half()).double().mean() < 0.01
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(2, 2, 64), (4, 1, 128), (6, 2, 128)])
+@pytest.mark.parametrize("first", [0, 50, 130])
+def test_values_that_are_not_finite(heads, kv_heads, head_dim, first):
+    """Infinities and NaNs of V reach the rows that see their positions, in their dimension, and no others; a row that sees an
+    infinity gets it and not the NaN that a zero weight, or a zero half of a weight, would make of it."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(first)
+    T = 90
+    q, k, v = (torch.randn(shape, generator=g, device="cuda").half()
+               for shape in [(T, heads, head_dim), (kv_heads, 256, head_dim), (kv_heads, 256, head_dim)])
+    v[:, first + 20, 3] = float("inf")
+    v[0, first + 21, 5] = float("-inf")
+    v[:, first + 41, 7] = float("nan")
+    v[-1, first + 70, 3] = float("-inf")
+    v[:, 220] = float("nan")  # past every row
+    scale = head_dim ** -0.5
+    got, want = _run(q, k, v, first, scale).double(), _exact(q, k, v, first, scale)
+    assert torch.isfinite(want[:20]).all() and not torch.isfinite(want[-1]).all()
+    assert (torch.isnan(got) == torch.isnan(want)).all()
+    assert (got[torch.isinf(want)] == want[torch.isinf(want)]).all()
+    ok = torch.isfinite(want)
+    assert ((got[ok] - want[ok]).abs() <= 2.0 ** -10.9 * want[ok].abs() + 2.0 ** -16).all()
+
+
+def test_keys_that_are_not_finite():
+    """A NaN or an infinity of K changes the rows that see it only."""
+    heads, kv_heads, head_dim, T, first = 4, 2, 64, 70, 10
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    q, k, v = (torch.randn(shape, generator=g, device="cuda").half()
+               for shape in [(T, heads, head_dim), (kv_heads, 128, head_dim), (kv_heads, 128, head_dim)])
+    scale = head_dim ** -0.5
+    clean = _run(q, k, v, first, scale)
+    for bad in (float("nan"), float("inf")):
+        k2 = k.clone()
+        k2[:, first + 33, 2] = bad
+        got = _run(q, k2, v, first, scale)
+        assert (got[:33] == clean[:33]).all()
+        assert torch.isnan(got[33:]).any()
