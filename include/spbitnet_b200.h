@@ -135,7 +135,7 @@ int spb_sparse_bitlinear_gemm(const uint32_t* meta, const uint32_t* values, cons
                               const float* d_absmax, float gamma, int32_t* acc_workspace, int rows, int cols,
                               int n, int meta_row_stride, int values_row_stride, void* stream);
 
-/* Which form spb_sparse_ternary_gemm uses: 0 (default) = automatic: up to 8 batch rows of matrices up to 40 M weights the
+/* Which form spb_sparse_ternary_gemm uses: 0 (default) = automatic: for few batch rows, where it measures faster, the
  * warp-level sparse MMA form (mma.sp m16n8k64, operands re-encoded in registers; needs cols % 256 == 0, row strides
  * that are multiples of 4 words and 16-byte aligned meta / values / X), else the tcgen05 sparse form
  * (tcgen05.mma.sp: sign bytes as the compressed operand, index pairs in tensor memory), which takes any layout;

@@ -5,9 +5,12 @@
 // for the group: tiles of 32 positions, two in flight.  A lane forms the score of one position, then holds head_dim / 32 of
 // the output's dims while the tile's weights go round by shuffles.  Scores, running maximum, sum and output are fp32.
 //
-// Bound: the caches through HBM for long sequences, the two barriers and one tile's chain for short ones.  One block per
-// (query head, sequence), a warp per position with 2-byte loads, used before: 23.5 us for 64 sequences of 16 positions at 64
-// heads of 128 over 8 KV heads; this form 7.7 us.
+// Bound: the caches through HBM with one query head per KV head and blocks enough (64 sequences of 4000 positions, 20 heads of
+// 128: 422 us, 6.2 TB/s); the arithmetic of a block's warps with groups (8 KV heads of 8: 578 us, 1.8 TB/s); a block's tiles one
+// after the other where KV heads times sequences leave SMs idle (two sequences of 4000 at 5 KV heads of 4: 141 us); two barriers
+// and one tile's chain for short sequences.  One block per (query head, sequence), a warp per position with 2-byte loads, used
+// before, was slower by 1.3 to 4.6 over 1, 2, 3, 4 and 8 heads per KV head, head dims 64 and 128, 2 to 64 sequences of 1 to 4000
+// positions: 1270, 2379 and 291 us for the three above, 24.2 against 6.2 for 64 sequences of 16 positions at 8 KV heads of 8.
 #include "fused_ops.cuh"
 
 namespace spb {

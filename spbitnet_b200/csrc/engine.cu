@@ -408,10 +408,10 @@ int ensure_graph(spb_engine* e, bool record_tokens, int n_prompt) {
 }
 
 // ---- batched prefill -------------------------------------------------------------------------------
-// T prompt tokens go through a layer together: the BitLinear layers run as the batched product
-// (spb_sparse_ternary_gemm, one activation row per token, integer-exact) followed by a per-row dequantise,
-// the vector ops as one block per token, attention as one block per (head, token) over the positions up to
-// the token's own.  Every rounding point of the token-serial step is kept, so the integer accumulators and
+// T prompt tokens go through a layer together: the BitLinear layers run as the batched product with the per-row
+// dequantise in its epilogue (bitlinear_gemm_group, one activation row per token, integer-exact; q, k and v and then
+// gate and up in one launch each), the vector ops as one block per token (row_ops.cu), attention on the tensor cores
+// (attention_prefill.cu; shapes that it does not take as one block per head and token).  Every rounding point of the token-serial step is kept, so the integer accumulators and
 // the quantised activations are the ones forward() produces token by token; only the attention sums are
 // formed in a different order (the split-KV kernel is not used here).
 

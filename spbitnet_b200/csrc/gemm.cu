@@ -2,11 +2,12 @@
 //
 // The reference has no kernel of its own for this; its batched path hands a dense
 // int8 copy of the weights to cuSPARSELt (src/cusparselt_backend.cu:186-207).  Here
-// the compressed format is consumed directly.  This file holds the SIMT form used
-// for small batches: every thread decodes its unit (128 columns of one row) once
-// into 32 packed int8x4 weight words held in registers and replays them against
-// kBatchTile activation rows staged in shared memory, so the weight stream is read
-// from HBM once per kBatchTile rows.
+// the compressed format is consumed directly.  This file chooses the form of a product
+// (gemm_mmasp.cu, gemm_tcsp_ws.cu) and holds the SIMT form, which only
+// spb_set_gemm_variant(1) asks for: every thread decodes its unit (128 columns of one
+// row) once into 32 packed int8x4 weight words held in registers and replays them
+// against kBatchTile activation rows staged in shared memory, so the weight stream is
+// read from HBM once per kBatchTile rows.
 #include "gemm_tcsp_ws.cuh"
 #include "spb_common.cuh"
 

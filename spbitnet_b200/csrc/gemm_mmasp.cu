@@ -7,8 +7,7 @@
 // in by 16-byte asynchronous copies, bitmap words are turned into index pairs and sign nibbles into
 // +1 / -1 bytes in registers, and the N = 8 columns of the instruction, which the GEMV fills with copies
 // of one vector, carry eight different activation rows here.  A warp re-encodes a step (64 columns of 16
-// rows) once and issues one MMA per tile of eight activation rows, so 8, 16, 24 or 32 rows cost little
-// more than one.  The reference has no kernel of its own for this (its batched path hands a dense copy
+// rows) once and issues one MMA per tile of eight activation rows.  The reference has no kernel of its own for this (its batched path hands a dense copy
 // to cuSPARSELt, src/cusparselt_backend.cu:186-207).
 //
 // Work split: a block of eight warps owns RB row blocks of 16 weight rows x KS warps, each warp a range of

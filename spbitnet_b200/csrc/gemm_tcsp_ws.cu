@@ -19,7 +19,7 @@
 // What bounds it.  An MMA of 64 columns takes 47 + N / 2 clocks.  With wide batches the tensor pipe and the activation
 // traffic out of L2 (256-row blocks halve it); with few batch rows the re-encoding, 650 clocks per step; below a dozen
 // steps per block the start of a block (2 us) and, with a split, the exchange at 13 B per clock and SM.
-//   28672 x 8192, n = 1024: 275 -> 129 us;  n = 64: 105 -> 23 us;  2560 x 6912, n = 200: 20.1 -> 9.7 us, against a form in
+//   28672 x 8192, n = 1024: 276 -> 147 us a call;  in a graph n = 64: 105 -> 25 us;  2560 x 6912, n = 200: 20.1 -> 9.7, against a form in
 //   which weights came by 16-byte loads of a row per lane (32 cache lines per instruction), signs through a table in shared
 //   memory, and the MMA thread divided four times per half step to find its ring slots (1050 of 1100 clocks).
 // A sign word of 32 weights becomes 32 bytes by a bit transpose and eight byte permutes whose selectors are the sign bits

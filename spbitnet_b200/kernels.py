@@ -52,7 +52,7 @@ def set_gemv_variant(variant: int) -> int:
 
 
 def set_gemm_variant(variant: int) -> int:
-    """0 automatic, 1 SIMT form, 2 tcgen05 tensor-core form."""
+    """0 automatic, 1 SIMT form, 3 tcgen05 sparse form, 4 warp-level sparse MMA form where it applies, else 3."""
     return load().spb_set_gemm_variant(int(variant))
 
 
