@@ -81,7 +81,18 @@ __device__ __noinline__ void pa_rows_one_by_one(const __half* __restrict__ Q, co
             float s = -INFINITY;
             if (p < n) {
                 s = 0.0f;
-                for (int d = 0; d < HD; ++d) s = fmaf(__half2float(q[d]), __half2float(K[static_cast<size_t>(p) * HD + d]), s);
+                const uint4* kr = reinterpret_cast<const uint4*>(K + static_cast<size_t>(p) * HD);
+#pragma unroll 4
+                for (int c = 0; c < HD / 8; ++c) {
+                    const uint4 kv = kr[c], qv = reinterpret_cast<const uint4*>(q)[c];
+                    const uint32_t kw[4] = {kv.x, kv.y, kv.z, kv.w}, qw[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&qw[i])), b = __half22float2(*reinterpret_cast<const __half2*>(&kw[i]));
+                        s = fmaf(a.x, b.x, s);
+                        s = fmaf(a.y, b.y, s);
+                    }
+                }
                 s *= scale_log2;
             }
             float mn = s;
@@ -93,7 +104,9 @@ __device__ __noinline__ void pa_rows_one_by_one(const __half* __restrict__ Q, co
             l = l * corr + e;
 #pragma unroll
             for (int i = 0; i < kDims; ++i) o[i] *= corr;
-            for (int r = 0; r < min(32, n - p0); ++r) {
+            const int seen = min(32, n - p0);
+#pragma unroll 4
+            for (int r = 0; r < seen; ++r) {
                 const float w = __shfl_sync(0xFFFFFFFFu, e, r);
 #pragma unroll
                 for (int i = 0; i < kDims; ++i) o[i] = fmaf(w, __half2float(V[static_cast<size_t>(p0 + r) * HD + 32 * i + lane]), o[i]);

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
             int issued = min(a.sw, nchunks);
             w.ph = 1;
             for (; issued < nchunks; ++issued, w.advance(a.sw)) {
-                if (!(ok = ws_wait(w_free + 8 * w.s, w.ph ^ 1u, a.wait_cycles))) break;
+                if (!(ok = ws_wait_dep(w_free + 8 * w.s, w.ph ^ 1u, a.wait_cycles))) break;
                 load_chunk(issued, w.s);
             }
             for (int c = max(0, issued - a.sw); c < issued; ++c)  // nothing in flight when the block leaves
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
             uint32_t abar = a_full, bbar = b_full;  // the matching "free" barriers lie 64 bytes on
             uint32_t aph = 0, bph = 0;
             auto half = [&](uint32_t h) {
-                if (!ws_wait(bbar, bph, a.wait_cycles)) return false;
+                if (!ws_wait_dep(bbar, bph, a.wait_cycles)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 ws_mma(tmem_d, a_lo + 4 * h, b_lo, idesc, acc, te + 4 * h);
                 ws_mma(tmem_d, a_lo + 4 * h + 2, b_lo + 4, idesc, 1, te + 4 * h + 2);
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(LAYOUT != kAny ? kWsThreadsTiled : kWsThreadsA
             ws_sign_bytes(vv.x, w0);
             ws_sign_bytes(vv.y, w1);
             const int sA = ca.s;
-            ok = ws_wait(a_free + 8 * sA, ca.ph ^ 1u, a.wait_cycles);
+            ok = ws_wait_dep(a_free + 8 * sA, ca.ph ^ 1u, a.wait_cycles);
             ok = __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;  // tcgen05.st below is warp-wide
             if (!ok) break;
             const uint32_t eaddr = tmem_e + lane_base + static_cast<uint32_t>((sA * a.mh + mhalf) * 8 + thalf * 4);

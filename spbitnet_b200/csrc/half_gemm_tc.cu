@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kHgThreads, 1) half_gemm_tc_kernel(const HgArg
             WsCursor c;
             uint32_t acc = 0;
             for (int k = 0; k < nk; ++k, c.advance(kHgStages)) {
-                if (!(ok = ws_wait(full + 8 * c.s, c.ph, kWsWaitCycles))) break;
+                if (!(ok = ws_wait_dep(full + 8 * c.s, c.ph, kWsWaitCycles))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t st = ring + c.s * stage;
                 const uint64_t w0 = ws_smem_desc(st), w1 = ws_smem_desc(st + kHgWBytes / 2), x = ws_smem_desc(st + kHgWBytes);

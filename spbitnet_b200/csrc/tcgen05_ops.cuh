@@ -48,6 +48,20 @@ __device__ __forceinline__ bool ws_wait(uint32_t mbar, uint32_t parity, long lon
         if (clock64() - t0 > limit) return false;
     }
 }
+// For what comes only after the grid's predecessors: their time does not count towards the bound.
+__device__ __forceinline__ bool ws_wait_dep(uint32_t mbar, uint32_t parity, long long limit) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    grid_dep_wait();
+    return ws_wait(mbar, parity, limit);
+}
 __device__ __forceinline__ void ws_arrive(uint32_t mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }

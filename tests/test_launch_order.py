@@ -33,3 +33,12 @@ def test_kernels_wait_for_their_predecessor():
     assert len(found) > 40 and WITHOUT_ATTRIBUTE <= set(found)
     missing = [n for n, body in found.items() if "grid_dep_wait()" not in body and n not in WITHOUT_ATTRIBUTE]
     assert not missing, missing
+
+
+def test_waits_behind_a_predecessor_are_bounded_from_its_end():
+    """Weights are on their way before a grid's predecessors are done; what follows from the activations comes after them, and their
+    time must not count towards the bound of such a wait."""
+    for name, barriers in {"gemm_tcsp_ws.cu": ["w_free + 8 * w.s", "bbar", "a_free + 8 * sA"], "half_gemm_tc.cu": ["full + 8 * c.s"]}.items():
+        text = (CSRC / name).read_text()
+        for b in barriers:
+            assert f"ws_wait_dep({b}," in text and f"ws_wait({b}," not in text, (name, b)
